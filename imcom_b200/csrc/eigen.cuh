@@ -37,6 +37,15 @@ int twostage_tridiag(imcom_ctx* ctx, DMat& Aw, DMat& Vall, double* d, double* e,
                      double* W, long long ldw, double* XY, void* scratch, long long spin);
 int twostage_backtransform2(imcom_ctx* ctx, int n, void* scratch, double* Z, long long ldz);
 
+// The end of the tridiagonalisation with the trailing matrix (rows and columns
+// k0 .. n-1) resident in the shared memory of `sms` SMs (eigen_res.cu):
+// largest trailing size, scratch bytes, and the launch.
+constexpr int RES_TRD_MAX = 2048;
+int resident_max(imcom_ctx* ctx, int sms);
+size_t resident_bytes(int n);
+int resident_tridiag(imcom_ctx* ctx, const DMat& Aw, DMat& Vall, double* d, double* e, double* tau,
+                     int k0, int sms, void* scratch, int* err, long long spin, int stall);
+
 // Keep-if-large-enough vector allocation.
 template <class T>
 inline int ensure_vec_keep(imcom_ctx* ctx, T** p, size_t& cap, size_t count) {

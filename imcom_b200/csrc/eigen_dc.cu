@@ -23,6 +23,8 @@
 //    product with K = 2 NB ([V W] [W V]^T), over the tiles on or below the
 //    diagonal (LAPACK dsyr2k 'L').
 //    Grid barriers spin with a bound and report a timeout instead of hanging.
+//    Once the trailing matrix fits the SMs' shared memory, eigen_res.cu
+//    factorises the rest.
 // 2. Divide and conquer (LAPACK dstedc / dlaed0-4 structure).  Leaves of at
 //    most 32 rows are diagonalised by a cyclic Jacobi sweep in one CTA each.
 //    Each merge level runs batched over all nodes: z vector and sort (merge
@@ -591,7 +593,8 @@ __global__ void __launch_bounds__(TRD_THREADS, 1) trd_panel_kernel(TrdArgs a) {
 }
 
 // ---------------------------------------------------------------------------
-// 1b. The last columns of the tridiagonalisation in one thread-block cluster.
+// 1b. The last columns of the tridiagonalisation in one thread-block cluster
+// (where IMCOM_OPT_TAIL_CTAS asks for one; by default eigen_res.cu takes over).
 //
 // Once the trailing matrix is small, every column of the panel kernel is a
 // chain of dependent L2 round trips and two grid barriers (~9 us whatever
@@ -1527,7 +1530,7 @@ static void tail_config(imcom_ctx* ctx, int* tail_ctas_out, int* tail_max_out) {
 static int sytrd_launches(imcom_ctx* ctx, DMat& Aw, DMat& Vall, double* d, double* e,
                           double* tau, double* W, long long ldw, double* ypart, double* ycol,
                           long long ldy, void* accbuf, long long spin, double* XY, int tail_ctas,
-                          int tail_max, bool capturing) {
+                          int tail_max, int res_max, void* resbuf, bool capturing) {
   const int n = (int)Aw.rows;
   int grid = sm_count(ctx);  // one CTA per SM: the cheapest grid barrier
   TrdAcc* acc = (TrdAcc*)accbuf;
@@ -1536,6 +1539,15 @@ static int sytrd_launches(imcom_ctx* ctx, DMat& Aw, DMat& Vall, double* d, doubl
   IMC_CUDA(cudaMemsetAsync(sync, 0, sizeof(GridSync), ctx->stream));
   bool tail_done = false;
   for (int k = 0; k < n - 1; k += NB) {
+    // the trailing matrix fits the SMs' shared memory: 3.7 us per column from
+    // 2048 down (2.0 us from 500), against 11 to 8 us on panels and 7.2 us in
+    // the cluster tail below
+    if (n - k <= res_max) {
+      IMC_TRY(resident_tridiag(ctx, Aw, Vall, d, e, tau, k, grid, resbuf, flag, spin,
+                               (ctx->stall_test & IMCOM_STALL_TRIDIAG) ? 1 : 0));
+      tail_done = true;
+      break;
+    }
     if (tail_ctas && n - k <= tail_max) {
       const int S = n - k;
       TailArgs ta{Aw.p, Aw.ld, Vall.p, Vall.ld, d, e, tau, n, k, (S + tail_ctas - 1) / tail_ctas};
@@ -1611,7 +1623,7 @@ static int sytrd_launches(imcom_ctx* ctx, DMat& Aw, DMat& Vall, double* d, doubl
 // direct path in place.
 static int sytrd_gpu(imcom_ctx* ctx, DMat& Aw, DMat& Vall, double* d, double* e, double* tau,
                      double* W, long long ldw, double* ypart, double* ycol, long long ldy,
-                     void* accbuf, long long spin, double* XY) {
+                     void* accbuf, long long spin, double* XY, void* resbuf) {
   const int n = (int)Aw.rows;
   int dev = ctx->device, coop = 0;
   cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
@@ -1628,7 +1640,8 @@ static int sytrd_gpu(imcom_ctx* ctx, DMat& Aw, DMat& Vall, double* d, double* e,
   if (per_sm < 1 || per_sm_c < 1)
     return set_err(ctx, IMCOM_ERR_CUDA, "panel kernel does not fit on an SM");
   int tail_ctas = 0, tail_max = 0;
-  tail_config(ctx, &tail_ctas, &tail_max);
+  const int res_max = ctx->tail_ctas == 0 ? resident_max(ctx, sm_count(ctx)) : 0;
+  if (!res_max) tail_config(ctx, &tail_ctas, &tail_max);
   GridSync* sync = (GridSync*)((char*)accbuf + 2 * sizeof(TrdAcc) + 64);
   EigWork* ew = eig_work(ctx);
   const long long key[] = {n, (long long)(uintptr_t)Aw.p, Aw.ld, (long long)(uintptr_t)Vall.p,
@@ -1636,7 +1649,8 @@ static int sytrd_gpu(imcom_ctx* ctx, DMat& Aw, DMat& Vall, double* d, double* e,
                            (long long)(uintptr_t)tau, (long long)(uintptr_t)W, ldw,
                            (long long)(uintptr_t)ypart, (long long)(uintptr_t)ycol, ldy,
                            (long long)(uintptr_t)accbuf, spin, (long long)(uintptr_t)XY,
-                           sm_count(ctx), tail_ctas, tail_max, ctx->stall_test};
+                           sm_count(ctx), tail_ctas, tail_max, ctx->stall_test, res_max,
+                           (long long)(uintptr_t)resbuf};
   constexpr int NKEY = (int)(sizeof(key) / sizeof(key[0]));
   static_assert(NKEY <= EigWork::kTrdKey, "graph key size");
   const bool same = std::equal(key, key + NKEY, ew->trd_key);
@@ -1660,7 +1674,7 @@ static int sytrd_gpu(imcom_ctx* ctx, DMat& Aw, DMat& Vall, double* d, double* e,
       int st = 0;
       if (ok) {
         st = sytrd_launches(ctx, Aw, Vall, d, e, tau, W, ldw, ypart, ycol, ldy, accbuf, spin,
-                            XY, tail_ctas, tail_max, true);
+                            XY, tail_ctas, tail_max, res_max, resbuf, true);
         ok = cudaStreamEndCapture(ctx->stream, &graph) == cudaSuccess && st == 0 && graph;
       }
     }
@@ -1676,11 +1690,11 @@ static int sytrd_gpu(imcom_ctx* ctx, DMat& Aw, DMat& Vall, double* d, double* e,
       ew->trd_graph_off = true;  // run directly from now on
       ctx->err.clear();
       IMC_TRY(sytrd_launches(ctx, Aw, Vall, d, e, tau, W, ldw, ypart, ycol, ldy, accbuf, spin,
-                             XY, tail_ctas, tail_max, false));
+                             XY, tail_ctas, tail_max, res_max, resbuf, false));
     }
   } else {
     IMC_TRY(sytrd_launches(ctx, Aw, Vall, d, e, tau, W, ldw, ypart, ycol, ldy, accbuf, spin, XY,
-                           tail_ctas, tail_max, false));
+                           tail_ctas, tail_max, res_max, resbuf, false));
   }
   // a timed-out grid barrier ends the factorisation with an error
   int h = 0;
@@ -1720,7 +1734,7 @@ int eigen_dc(imcom_ctx* ctx, const DMat& A, DMat& Wout, double* wout) {
   size_t o_d = take(n * 8), o_e = take(n * 8), o_tau = take(n * 8), o_dt = take(n * 8);
   size_t o_W = take((size_t)ldw * NB * 8), o_y = take((size_t)ldy * (nch + nrb) * 8);
   size_t o_XY = take((size_t)ldw * 4 * NB * 8);
-  size_t o_acc = take(4096);
+  size_t o_acc = take(4096), o_res = take(resident_bytes(n));
   size_t o_split = take((size_t)n * 4), o_nodes = take((size_t)n * sizeof(Node));
   size_t o_wk = take(((size_t)n * 8 + 16) * 9 + ((size_t)n * 4 + 16) * 8 + ((size_t)n * 24 + 32) +
                      4096);
@@ -1757,7 +1771,7 @@ int eigen_dc(imcom_ctx* ctx, const DMat& A, DMat& Wout, double* wout) {
                              base + o_2s, spin));
   else
     IMC_TRY(sytrd_gpu(ctx, Aw, Vall, d, e, tau, Wp, ldw, yp, yp + (size_t)ldy * nch, ldy,
-                      base + o_acc, spin, (double*)(base + o_XY)));
+                      base + o_acc, spin, (double*)(base + o_XY), base + o_res));
   stage_end(ctx, ST_EIG_TRD);
   stage_begin(ctx, ST_EIG_DC);
 

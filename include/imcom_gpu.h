@@ -91,13 +91,14 @@ typedef struct imcom_ctx imcom_ctx;
  * the same time on one GPU each take a share.  Results agree to rounding
  * (the reduction order of the eigensolver follows the grid). */
 #define IMCOM_OPT_SM_SHARE 10
-/* Thread-block cluster that finishes the tridiagonalisation once the
- * trailing matrix fits its distributed shared memory: 0 = automatic (16 CTAs
- * where the device can place them, else 8), 8 or 16 = that many CTAs (8 if 16
- * cannot be placed), -1 = no cluster tail (panels to the end).  A 16-CTA
- * cluster must find 16 free SMs in one GPC, which contexts working side by
- * side can make wait; smaller clusters hold smaller tails.  Same results to
- * rounding either way. */
+/* How the tridiagonalisation ends: 0 (default) = the trailing matrix resident
+ * in the shared memory of this context's SMs (up to order 2048 on 148 SMs),
+ * one exchange per column; 8 or 16 = a thread-block cluster of that many
+ * CTAs (8 if 16 cannot be placed) once the trailing matrix fits its
+ * distributed shared memory; -1 = panels to the end.  A 16-CTA cluster must
+ * find 16 free SMs in one GPC, which contexts working side by side can make
+ * wait; smaller clusters hold smaller tails.  Same results to rounding
+ * either way. */
 #define IMCOM_OPT_TAIL_CTAS 11
 /* Kernel of imcom_gpu_build_images: 0 = the FP64 GEMM, 1 = a streaming
  * kernel for a few stacks (up to 8 stacks per pass over T, FP64 FMA, each
@@ -148,10 +149,10 @@ typedef struct imcom_ctx imcom_ctx;
  *    (bounded at 2 s) runs out; the kernel drains, frees its tensor memory
  *    and returns, and the next bisection returns IMCOM_ERR_SPLIT;
  *  IMCOM_STALL_TRIDIAG: the first grid barrier of the tridiagonalisation
- *    waits for one arrival more than the grid makes, so it gives up after
- *    IMCOM_OPT_EIGEN_MAXITER polls and imcom_gpu_eigen_A returns
- *    IMCOM_ERR_EIGEN (when the tridiagonalisation runs panels: n above the
- *    cluster tail's size, or IMCOM_OPT_TAIL_CTAS = -1).
+ *    waits for one arrival more than the grid makes (or, where no panel runs,
+ *    the first exchange of the resident columns for a value that nobody
+ *    publishes), so it gives up after IMCOM_OPT_EIGEN_MAXITER polls and
+ *    imcom_gpu_eigen_A returns IMCOM_ERR_EIGEN (not in the cluster tail).
  * The context stays usable: clear the option and the next call runs
  * normally. */
 #define IMCOM_OPT_STALL_TEST 16
