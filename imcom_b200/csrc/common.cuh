@@ -262,6 +262,9 @@ int dgemm(imcom_ctx* ctx, char transA, char transB, long long M, long long N,
           const double* B, long long ldb, double beta, double* C,
           long long ldc);
 
+// H (m x S) = T^T I for S image stacks on the tensor path (stacks.cu).
+int stacks_mma(imcom_ctx* ctx, int S, const double* dI, long long ldi, double* dH, long long ldh);
+
 int eigen_dc(imcom_ctx* ctx, const DMat& A, DMat& W, double* w);
 
 // Split-precision products (ozaki.cu).  split_operand slices the operand

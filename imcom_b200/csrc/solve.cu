@@ -447,10 +447,19 @@ static int launch_stacks(imcom_ctx* ctx, int nstack, const double* dI, long long
 static int build_images(imcom_ctx* ctx, int nstack, const double* dI, long long ldi,
                         double* dH, long long ldh) {
   stage_begin(ctx, ST_EPI);
-  // the streaming kernel passes over T once per 8 stacks (~45 us each at
-  // n = m = 4096), the GEMM's time is flat at ~215 us up to 64 stacks
-  const bool stream = ctx->stack_kernel == IMCOM_STACKS_STREAM ||
-                      (ctx->stack_kernel == IMCOM_STACKS_AUTO && nstack <= IMCOM_STACKS_STREAM_MAX);
+  // Automatic: the tensor kernel for up to 64 stacks (one read of T), and for
+  // more while the product is small; above that the 128-wide GEMM tile is
+  // full enough.  Measured, tensor kernel / GEMM, us: 61 / 63 at n = 4096, m =
+  // 800, 128 stacks (4.2e8 products), 76 / 73 at m = 1200, 96 stacks (4.7e8),
+  // 223 / 178 at m = 4096, 128 stacks; the other way round 41 / 53 at n =
+  // 1000, m = 1500, 192 stacks (2.9e8).
+  if (ctx->stack_kernel == IMCOM_STACKS_AUTO &&
+      (nstack <= 64 || (double)ctx->n * ctx->m * nstack <= 3e8)) {
+    IMC_TRY(stacks_mma(ctx, nstack, dI, ldi, dH, ldh));
+    stage_end(ctx, ST_EPI);
+    return 0;
+  }
+  const bool stream = ctx->stack_kernel == IMCOM_STACKS_STREAM;
   if (stream) {
     // passes of at most 8 stacks: 4 x 8 partial sums and two 4 x 4 blocks of
     // T values per lane fill the register budget of three CTAs per SM

@@ -1,0 +1,220 @@
+// stacks.cu -- H = T^T I for several image stacks on the FP64 tensor path
+// (imcom_build_image, imcom_matrix.f90:754-790, for S stacks that share T).
+//
+// T (n x m) and the stacks (n x S) are both contiguous along the summed
+// dimension.  A CTA owns 32 output pixels and NT stacks; its eight warps are
+// 2 (pixels) x 4 (slices of each 64-deep stage), a warp holding 16 x NT sums
+// in m16n8k4 DMMA tiles, and the four slices are added through shared memory
+// at the end.  So T crosses HBM once for up to 64 stacks, the stacks come
+// from L2, and 32 pixels per CTA give one CTA per SM at m of about 4700
+// without splitting the sum; other sizes split it over a few CTAs and add the
+// partial sums in a second kernel.
+//
+// What bounds it: HBM (one read of T) up to about 16 stacks, the FP64 tensor
+// pipe above.  The 128 x 128 GEMM tile computes 128 stacks whatever S is, and
+// the FMA kernel (solve.cu) reads T once per eight stacks and is bound by its
+// shared-memory reads.  Measured, n = m = 4096, three T in turn (402 MB), us:
+//   S        1      8     16     48     64    128
+//   GEMM   143    143    143    144    145    149
+//   FMA     22     38     73    199    274    517
+//   here  19.4   19.6   25.3   64.9   77.8    155
+// (48 stacks are 1.6 GFLOP, 45 us at the DGEMM rate.)  Issuing a stage's
+// copies before its products instead of between them: 77.0 at S = 48; twice
+// the warps: 81.7.
+#include <algorithm>
+
+#include "common.cuh"
+#include "dgemm_tile.cuh"
+
+namespace imcom {
+
+__global__ void splitk_reduce_kernel(const double* __restrict__ part, long long ldp, int splits,
+                                     long long M, long long N, double alpha, double beta,
+                                     double* __restrict__ C, long long ldc);
+
+namespace {
+
+constexpr int ST_THREADS = 256, ST_BM = 32, ST_BK = 64;
+constexpr int ST_WM = 2, ST_WK = 4;        // warps over pixels and over each stage's depth
+constexpr int ST_SK = ST_BK + 4;           // shared stride: fragment loads hit distinct banks
+constexpr int ST_KW = ST_BK / ST_WK;       // depth per warp and stage
+
+template <int NT>
+constexpr int st_stage() {
+  return (ST_BM + NT) * ST_SK;
+}
+// Stages in flight: four, or what fits with the sums' exchange area.
+template <int NT>
+constexpr int st_stages() {
+  return NT <= 32 ? 4 : 3;
+}
+template <int NT>
+constexpr size_t st_smem() {
+  const size_t pipe = (size_t)st_stages<NT>() * st_stage<NT>();
+  const size_t sums = (size_t)ST_WK * ST_BM * (NT + 1);
+  return (pipe > sums ? pipe : sums) * sizeof(double);
+}
+
+// VI: doubles per copy of the stacks (2 where their columns are 16-byte
+// aligned, else 1); T's columns always are.
+template <int NT, int VI>
+__global__ void __launch_bounds__(ST_THREADS)
+stacks_mma_kernel(const double* __restrict__ T, long long ldt, const double* __restrict__ I,
+                  long long ldi, double* __restrict__ H, long long ldh, int n, int m, int S,
+                  int kchunk) {
+  extern __shared__ __align__(16) double st_sm[];
+  constexpr int STG = st_stages<NT>(), SZ = st_stage<NT>();
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int wm = warp & (ST_WM - 1), wk = warp / ST_WM;
+  const int g = lane >> 2, t = lane & 3;
+  const int a0 = blockIdx.x * ST_BM, s0 = blockIdx.y * NT;
+  const int kb = blockIdx.z * kchunk, ke = min(n, kb + kchunk);
+  const int nk = (ke - kb + ST_BK - 1) / ST_BK;
+  const int na = min(ST_BM, m - a0), ns = min(NT, S - s0);
+  T += (long long)a0 * ldt;
+  I += (long long)s0 * ldi;
+  if (gridDim.z > 1) H += (size_t)blockIdx.z * (size_t)ldh * (size_t)S;  // partial slice
+
+  // Quarter u of stage kt: pixel rows 8 u .. 8 u + 7 of T and every fourth
+  // group of the stacks' copies.
+  const int tr = tid / (ST_BK / 2), tk = tid % (ST_BK / 2) * 2;
+  const double* tsrc = T + (long long)tr * ldt + kb + tk;
+  double* tdst = st_sm + tr * ST_SK + tk;
+  const int ir = tid / (ST_BK / VI), ik = tid % (ST_BK / VI) * VI;
+  constexpr int IROWS = ST_THREADS / (ST_BK / VI);  // stacks per group of copies
+  const double* isrc = I + (long long)ir * ldi + kb + ik;
+  double* idst = st_sm + (ST_BM + ir) * ST_SK + ik;
+  auto load = [&](int kt, int u) {
+    const int st = (kt % STG) * SZ, left = ke - kb - kt * ST_BK;
+    {
+      const int r = tr + 8 * u, l = r < na ? left - tk : 0;
+      gemm::cp_async(tdst + st + 8 * u * ST_SK,
+                     l > 0 ? tsrc + (long long)8 * u * ldt + kt * ST_BK : T,
+                     8 * max(0, min(l, 2)), 2);
+    }
+#pragma unroll
+    for (int q = u; q < NT / IROWS; q += 4) {
+      const int r = ir + IROWS * q, l = r < ns ? left - ik : 0;
+      gemm::cp_async(idst + st + IROWS * q * ST_SK,
+                     l > 0 ? isrc + (long long)IROWS * q * ldi + kt * ST_BK : I,
+                     8 * max(0, min(l, VI)), VI);
+    }
+  };
+  static_assert(ST_BM == 32 && ST_THREADS / (ST_BK / 2) == 8 && ST_KW == 16, "quarters of a stage");
+
+  double acc[NT / 8][4];
+#pragma unroll
+  for (int j = 0; j < NT / 8; ++j)
+#pragma unroll
+    for (int r = 0; r < 4; ++r) acc[j][r] = 0.0;
+#pragma unroll
+  for (int s = 0; s < STG - 1; ++s) {
+    if (s < nk)
+      for (int u = 0; u < 4; ++u) load(s, u);
+    gemm::cp_commit();
+  }
+  for (int kt = 0; kt < nk; ++kt) {
+    gemm::cp_wait<STG - 2>();
+    __syncthreads();
+    const double* sa = st_sm + (kt % STG) * SZ + (wm * 16 + g) * ST_SK + wk * ST_KW + t;
+    const double* sb = st_sm + (kt % STG) * SZ + (ST_BM + g) * ST_SK + wk * ST_KW + t;
+#pragma unroll
+    for (int kk = 0; kk < ST_KW; kk += 4) {
+      // the next stage's copies between the products, which leave most issue
+      // slots free
+      if (kt + STG - 1 < nk) load(kt + STG - 1, kk / 4);
+      const double f0 = sa[kk], f1 = sa[8 * ST_SK + kk];
+#pragma unroll
+      for (int j = 0; j < NT / 8; ++j) {
+        const double b = sb[8 * j * ST_SK + kk];
+        asm volatile(
+            "mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5}, {%6}, "
+            "{%0,%1,%2,%3};\n"
+            : "+d"(acc[j][0]), "+d"(acc[j][1]), "+d"(acc[j][2]), "+d"(acc[j][3])
+            : "d"(f0), "d"(f1), "d"(b));
+      }
+    }
+    gemm::cp_commit();
+  }
+  gemm::cp_wait<0>();
+  __syncthreads();
+  // the four depth slices' sums, [slice][pixel][stack]
+  double* sums = st_sm + (size_t)wk * ST_BM * (NT + 1);
+#pragma unroll
+  for (int j = 0; j < NT / 8; ++j)
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+      sums[(wm * 16 + g + ((r >> 1) ? 8 : 0)) * (NT + 1) + 8 * j + 2 * t + (r & 1)] = acc[j][r];
+  __syncthreads();
+  for (int e = tid; e < ST_BM * NT; e += ST_THREADS) {
+    const int r = e % ST_BM, s = e / ST_BM;
+    if (r < na && s < ns) {
+      const double* p = st_sm + r * (NT + 1) + s;
+      constexpr int Z = ST_BM * (NT + 1);
+      H[(a0 + r) + (long long)(s0 + s) * ldh] = (p[0] + p[Z]) + (p[2 * Z] + p[3 * Z]);
+    }
+  }
+}
+
+template <int NT>
+int launch_nt(imcom_ctx* ctx, int S, const double* dI, long long ldi, double* dH, long long ldh) {
+  const int n = ctx->n, m = ctx->m, sms = sm_count(ctx);
+  const long long tiles = (long long)((m + ST_BM - 1) / ST_BM) * ((S + NT - 1) / NT);
+  // slices of the sum: the fewest rounds of stages per SM, each further slice
+  // charged with the second kernel (about 3 us, 12 stages) and its partial
+  // sums (about 2 stages per million)
+  const int ksteps = (n + ST_BK - 1) / ST_BK;
+  int splits = 1;
+  double best = 0.0;
+  for (int s = 1; s <= 16 && ksteps >= 4 * s; ++s) {
+    double cost = (double)((tiles * s + sms - 1) / sms) * ((ksteps + s - 1) / s);
+    if (s > 1) cost += 12.0 + 2e-6 * s * (double)m * S;
+    if (s == 1 || cost < best) {
+      best = cost;
+      splits = s;
+    }
+  }
+  const int kchunk = (ksteps + splits - 1) / splits * ST_BK;
+  splits = (n + kchunk - 1) / kchunk;
+  double* out = dH;
+  long long ldo = ldh;
+  if (splits > 1) {
+    ldo = pad_ld(m);
+    IMC_TRY(ensure_buf(ctx, &ctx->gemm_ws, ctx->gemm_ws_bytes,
+                       (size_t)splits * (size_t)ldo * (size_t)S * sizeof(double)));
+    out = (double*)ctx->gemm_ws;
+  }
+  const bool v2 = ((uintptr_t)dI & 15) == 0 && ldi % 2 == 0;
+  auto k = v2 ? stacks_mma_kernel<NT, 2> : stacks_mma_kernel<NT, 1>;
+  IMC_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)st_smem<NT>()));
+  const dim3 grd((unsigned)((m + ST_BM - 1) / ST_BM), (unsigned)((S + NT - 1) / NT),
+                 (unsigned)splits);
+  k<<<grd, ST_THREADS, st_smem<NT>(), ctx->stream>>>(ctx->T.p, ctx->T.ld, dI, ldi, out, ldo, n, m,
+                                                     S, kchunk);
+  IMC_LAUNCH();
+  if (splits > 1) {
+    const dim3 g2((unsigned)std::min((m + 255) / 256, 64), (unsigned)S);
+    splitk_reduce_kernel<<<g2, 256, 0, ctx->stream>>>(out, ldo, splits, m, S, 1.0, 0.0, dH, ldh);
+    IMC_LAUNCH();
+  }
+  return 0;
+}
+
+}  // namespace
+
+int stacks_mma(imcom_ctx* ctx, int S, const double* dI, long long ldi, double* dH,
+               long long ldh) {
+  // the narrowest tile that takes the stacks in the fewest reads of T
+  const int passes = (S + 63) / 64, per = (S + passes - 1) / passes;
+  if (per <= 8) return launch_nt<8>(ctx, S, dI, ldi, dH, ldh);
+  if (per <= 16) return launch_nt<16>(ctx, S, dI, ldi, dH, ldh);
+  if (per <= 24) return launch_nt<24>(ctx, S, dI, ldi, dH, ldh);
+  if (per <= 32) return launch_nt<32>(ctx, S, dI, ldi, dH, ldh);
+  if (per <= 40) return launch_nt<40>(ctx, S, dI, ldi, dH, ldh);
+  if (per <= 48) return launch_nt<48>(ctx, S, dI, ldi, dH, ldh);
+  if (per <= 56) return launch_nt<56>(ctx, S, dI, ldi, dH, ldh);
+  return launch_nt<64>(ctx, S, dI, ldi, dH, ldh);
+}
+
+}  // namespace imcom

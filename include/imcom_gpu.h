@@ -102,15 +102,16 @@ typedef struct imcom_ctx imcom_ctx;
 #define IMCOM_OPT_TAIL_CTAS 11
 /* Kernel of imcom_gpu_build_images: 0 = the FP64 GEMM, 1 = a streaming
  * kernel for a few stacks (up to 8 stacks per pass over T, FP64 FMA, each
- * warp holding four columns of T against the stacks of its pass), 2 = the
- * streaming kernel up to IMCOM_STACKS_STREAM_MAX stacks and the GEMM above
- * (default).  Same sums to rounding. */
+ * warp holding four columns of T against the stacks of its pass), 2 (default)
+ * = an FP64 tensor-core kernel with 32-pixel tiles for up to 64 stacks (and
+ * for more where the product is small), the GEMM above.  Same sums to
+ * rounding. */
 #define IMCOM_OPT_STACK_KERNEL 12
 #define IMCOM_STACKS_GEMM 0
 #define IMCOM_STACKS_STREAM 1
-#define IMCOM_STACKS_AUTO 2      /* default: streaming up to IMCOM_STACKS_STREAM_MAX
-                                   stacks, the GEMM above (measured crossover) */
-#define IMCOM_STACKS_STREAM_MAX 32
+#define IMCOM_STACKS_AUTO 2
+#define IMCOM_STACKS_STREAM_MAX 32 /* stacks beyond which the streaming kernel loses
+                                   to the GEMM */
 /* Inverse 2-D FFT of the lookup tables (imcom_build_Alookup/Blookup): 0 =
  * embedding, cuFFT and shift as separate steps; 1 = the library's own
  * transform in two passes that skip the grid's zero lines and fuse the
@@ -277,8 +278,8 @@ int imcom_gpu_build_image(imcom_ctx* ctx, double* H_out);
  * and PSFs of the resident T (built, or loaded from the cache with
  * imcom_gpu_load_T): column s of I_stack (n x nstack, leading dimension n) is
  * the I_i vector of stack s, column s of H_out (m x nstack, leading
- * dimension m) its H_a.  One FP64 GEMM H = T^T I, so T is read from HBM once
- * for all stacks.  Host arrays; H_out may be NULL (result kept on the
+ * dimension m) its H_a.  One FP64 product H = T^T I, so T is read from HBM
+ * once for up to 64 stacks.  Host arrays; H_out may be NULL (result kept on the
  * device). */
 int imcom_gpu_build_images(imcom_ctx* ctx, int nstack, const double* I_stack, double* H_out);
 /* The same on device arrays the caller owns (dI: n x nstack with leading
