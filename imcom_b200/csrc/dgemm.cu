@@ -11,7 +11,10 @@
 // Operands stream through a 3-stage cp.async shared-memory pipeline (216 KB,
 // one CTA per SM, one barrier per 32 of K); the shared layouts are padded so
 // every fragment load is bank-conflict free (stride 36 doubles for
-// k-contiguous tiles, 132 for m/n-contiguous ones).
+// k-contiguous tiles, 132 for m/n-contiguous ones).  A stage's copies are
+// issued between the products of the stage before it.  Bound by the DMMA
+// pipe: 34.1 TFLOP/s at 4096^3 (31.2 with the copies after the products;
+// cuBLAS 35.5, 37.2 from 64 FMA per clock and SM).
 #include <algorithm>
 
 #include "common.cuh"

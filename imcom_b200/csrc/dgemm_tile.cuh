@@ -26,38 +26,45 @@ __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_grou
 template <int N>
 __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N)); }
 
-// Load one operand tile.  KCONTIG: element (r, k) at P[k + r * ld] (r = m or
-// n), stored S[r][k] (stride SKC).  Otherwise element (r, k) at P[r + k * ld],
-// stored S[k][r] (stride SMC).  Out-of-range elements are zero-filled.
+// One operand tile.  KCONTIG: element (r, k) at P[k + r * ld] (r = m or n),
+// stored S[r][k] (stride SKC).  Otherwise element (r, k) at P[r + k * ld],
+// stored S[k][r] (stride SMC).  Out-of-range elements are zero-filled.  The
+// copies of a stage come in BK / 4 pieces, which the main loop issues between
+// its products; piece q of thread t is row (or k) t / PER + ROWS q.
 template <bool KCONTIG, int VEC>
-__device__ __forceinline__ void load_tile(double* S, const double* __restrict__ P, long long ld,
-                                          long long r0, long long k0, long long R, long long K) {
-  constexpr int CHUNKS = BM * BK / VEC;
-  for (int c = threadIdx.x; c < CHUNKS; c += THREADS) {
-    long long r, k;
-    double* dst;
-    int valid;
-    const double* src;
-    if (KCONTIG) {
-      constexpr int PER = BK / VEC;
-      int rr = c / PER, kk = (c % PER) * VEC;
-      r = r0 + rr;
-      k = k0 + kk;
-      dst = S + rr * SKC + kk;
-      valid = (r < R) ? (int)min((long long)VEC, max(0LL, K - k)) : 0;
-      src = valid ? P + k + r * ld : P;
-    } else {
-      constexpr int PER = BM / VEC;
-      int kk = c / PER, rr = (c % PER) * VEC;
-      r = r0 + rr;
-      k = k0 + kk;
-      dst = S + kk * SMC + rr;
-      valid = (k < K) ? (int)min((long long)VEC, max(0LL, R - r)) : 0;
-      src = valid ? P + r + k * ld : P;
-    }
-    cp_async(dst, src, valid * 8, VEC);
+struct TileLoad {
+  static constexpr int PER = (KCONTIG ? BK : BM) / VEC;  // copies per row (or k)
+  static constexpr int ROWS = THREADS / PER;             // rows (or k) per round of copies
+  static constexpr int ROUNDS = (KCONTIG ? BM : BK) / ROWS;
+  static constexpr int PIECE = ROUNDS / (BK / 4);        // rounds per piece
+  static_assert(THREADS % PER == 0 && ROUNDS % (BK / 4) == 0, "pieces of a stage");
+  const double* base;  // this thread's first element of stage 0
+  const double* P;
+  long long ld;
+  int dst, i0, o0, nrow;  // offset in the tile; own row (or k) and k (or row); rows in range
+
+  __device__ __forceinline__ TileLoad(const double* P_, long long ld_, long long r0, long long k0,
+                                      long long R) {
+    P = P_;
+    ld = ld_;
+    i0 = threadIdx.x / PER;
+    o0 = threadIdx.x % PER * VEC;
+    dst = i0 * (KCONTIG ? SKC : SMC) + o0;
+    base = KCONTIG ? P + (k0 + o0) + (r0 + i0) * ld : P + (r0 + o0) + (k0 + i0) * ld;
+    nrow = (int)min((long long)BM, R - r0);
   }
-}
+  // piece q of the stage at depth kt BK, with `left` = K minus that depth
+  __device__ __forceinline__ void piece(double* S, int kt, int left, int q) const {
+    const double* src = base + (long long)kt * BK * (KCONTIG ? 1 : ld);
+#pragma unroll
+    for (int u = 0; u < PIECE; ++u) {
+      const int i = (q * PIECE + u) * ROWS;
+      const int v = KCONTIG ? (i0 + i < nrow ? min(VEC, left - o0) : 0)
+                            : (i0 + i < left ? min(VEC, nrow - o0) : 0);
+      cp_async(S + dst + i * (KCONTIG ? SKC : SMC), v > 0 ? src + i * ld : P, 8 * max(v, 0), VEC);
+    }
+  }
+};
 
 // LOWER: only output tiles with a row on or below the diagonal (row >= col)
 // are computed; tiles strictly above it are left as they are (the symmetric
@@ -107,11 +114,17 @@ __device__ __forceinline__ void dgemm_tile(long long M, long long N, long long K
   auto stageA = [&](int s) { return smem + s * STAGE_DBL; };
   auto stageB = [&](int s) { return smem + s * STAGE_DBL + TILE_DBL; };
 
+  const TileLoad<AK, VEC> la(A, lda, m0, kb, M);
+  const TileLoad<BKC, VEC> lb(B, ldb, n0, kb, N);
+  const int klen = (int)(ke - kb);
 #pragma unroll
   for (int s = 0; s < STAGES - 1; ++s) {
     if (s < nk) {
-      load_tile<AK, VEC>(stageA(s), A, lda, m0, kb + (long long)s * BK, M, ke);
-      load_tile<BKC, VEC>(stageB(s), B, ldb, n0, kb + (long long)s * BK, N, ke);
+#pragma unroll 1
+      for (int q = 0; q < BK / 4; ++q) {
+        la.piece(stageA(s), s, klen - s * BK, q);
+        lb.piece(stageB(s), s, klen - s * BK, q);
+      }
     }
     cp_commit();
   }
@@ -121,8 +134,19 @@ __device__ __forceinline__ void dgemm_tile(long long M, long long N, long long K
     __syncthreads();
     const double* As = stageA(kt % STAGES);
     const double* Bs = stageB(kt % STAGES);
+    double* An = stageA((kt + STAGES - 1) % STAGES);
+    double* Bn = stageB((kt + STAGES - 1) % STAGES);
+    const bool more = kt + STAGES - 1 < nk;
+    const int lnext = klen - (kt + STAGES - 1) * BK;
 #pragma unroll
     for (int kk = 0; kk < BK; kk += 4) {
+      // a piece of the next stage's copies between the products: issued all
+      // together after them they cost a tenth of the main loop (both warps of
+      // a scheduler leave the tensor pipe idle meanwhile)
+      if (more) {
+        la.piece(An, kt + STAGES - 1, lnext, kk / 4);
+        lb.piece(Bn, kt + STAGES - 1, lnext, kk / 4);
+      }
       double af[4][2], bf[4];
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
@@ -149,11 +173,6 @@ __device__ __forceinline__ void dgemm_tile(long long M, long long N, long long K
               "{%0,%1,%2,%3};\n"
               : "+d"(acc[i][j][0]), "+d"(acc[i][j][1]), "+d"(acc[i][j][2]), "+d"(acc[i][j][3])
               : "d"(af[i][0]), "d"(af[i][1]), "d"(bf[j]));
-    }
-    int nxt = kt + STAGES - 1;
-    if (nxt < nk) {
-      load_tile<AK, VEC>(stageA(nxt % STAGES), A, lda, m0, kb + (long long)nxt * BK, M, ke);
-      load_tile<BKC, VEC>(stageB(nxt % STAGES), B, ldb, n0, kb + (long long)nxt * BK, N, ke);
     }
     cp_commit();
   }
