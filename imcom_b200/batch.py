@@ -3,17 +3,17 @@
 The reference solves one patch (one input stack, one output grid) per program
 run (imcom.f90:90-169).  A survey is processed as many such patches, and a
 patch of a few thousand input pixels leaves a B200 mostly idle: its
-eigensolver is a chain of dependent, latency-bound steps (one grid barrier
-pair per Householder column).  Here K worker threads each own a context
+eigensolver is a chain of dependent, latency-bound steps (one or two
+exchanges between its SMs per Householder column).  Here K worker threads each own a context
 (own CUDA stream, own buffers) whose persistent and cooperative kernels are
 sized for a share of the SMs (IMCOM_OPT_SM_SHARE), so K patches advance at
 once and their kernels fill the GPU together.  Patches are dealt from a
 queue, largest n first.
 
 `autotune` measures the patch throughput of candidate configurations --
-concurrency x the thread-block cluster that finishes each tridiagonalisation
-(IMCOM_OPT_TAIL_CTAS: 16 CTAs hold the longest tail but need 16 free SMs of
-one GPC, which contexts working side by side can make wait) -- on a sample of
+concurrency x what finishes each tridiagonalisation (IMCOM_OPT_TAIL_CTAS: the
+shared memory of the context's SMs, or a thread-block cluster, whose 16 CTAs
+need 16 free SMs of one GPC, which contexts working side by side can make wait) -- on a sample of
 the batch and returns the fastest (cached per GPU and size class).
 
 Results per patch are those of `Solver.solve` (K, U/S maps, H, the

@@ -244,6 +244,7 @@ void stage_end(imcom_ctx* ctx, Stage s);
 
 // Number of SMs of the context's device (cached).
 int sm_count(imcom_ctx* ctx);
+int device_sm_count(int device);
 
 // ---- kernels exported between translation units ----
 // FP64 GEMM: C (M x N) = alpha * op(A) * op(B) + beta * C, column-major.

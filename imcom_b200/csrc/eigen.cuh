@@ -37,6 +37,19 @@ int twostage_tridiag(imcom_ctx* ctx, DMat& Aw, DMat& Vall, double* d, double* e,
                      double* W, long long ldw, double* XY, void* scratch, long long spin);
 int twostage_backtransform2(imcom_ctx* ctx, int n, void* scratch, double* Z, long long ldz);
 
+// One panel of the tridiagonalisation (eigen_panel.cu): columns k .. k + b - 1
+// of the trailing matrix of Aw on G SMs, b at most TRD_NB.  panel_grid is the G
+// for order n (the context's SMs, or the fewest more whose CTAs' rows fit
+// their shared memory); panel_prepare sets the kernels' attributes (before any
+// stream capture); the scratch of panel_bytes starts zeroed.
+constexpr int TRD_NB = 32;
+int panel_grid(imcom_ctx* ctx, int n);
+size_t panel_bytes(int n, int G);
+int panel_prepare(imcom_ctx* ctx);
+int panel_launch(imcom_ctx* ctx, const DMat& Aw, DMat& Vall, double* W, long long ldw, double* d,
+                 double* e, double* tau, int k, int b, int G, void* scratch, int* err,
+                 long long spin, int stall);
+
 // The end of the tridiagonalisation with the trailing matrix (rows and columns
 // k0 .. n-1) resident in the shared memory of `sms` SMs (eigen_res.cu):
 // largest trailing size, scratch bytes, and the launch.

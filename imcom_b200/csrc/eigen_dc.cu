@@ -5,25 +5,11 @@
 // reversed by the caller (imcom_matrix.f90:656-662).
 //
 // 1. Tridiagonalisation (LAPACK dsytrd/dlatrd, lower).  Panels of NB = 32
-//    columns; only the lower triangle of the trailing matrix is read or
-//    updated.  Inside a panel every column needs the trailing symmetric
-//    matrix-vector product y0 = A22 v and the panel corrections
-//    y = y0 - V (W^T v) - W (V^T v).  One persistent cooperative kernel per
-//    panel runs the whole panel with two grid-wide barriers per column:
-//      phase A: A22 x for the raw column x = A(j+1:n, j) (so the tiles need
-//               not wait for the reflector), from 64 x 16 lower-triangle
-//               tiles staged through shared memory by cp.async: row sums
-//               and column sums per tile, and x^T A22 x (one atomic per CTA);
-//      phase B: y0 = scl A22 x + delta A22(:, j+1) for v = scl x +
-//               delta e_{j+1}, then w = tau (y - 1/2 tau (y^T v) v) row by
-//               row, using v^T y = v^T y0 - 2 (V^T v).(W^T v), the update of
-//               the next column, its norm and its dot products with the
-//               panel's W and V (the rows already hold them in registers).
-//    The trailing update A22 -= V W^T + W V^T runs on the DMMA GEMM as one
-//    product with K = 2 NB ([V W] [W V]^T), over the tiles on or below the
-//    diagonal (LAPACK dsyr2k 'L').
-//    Grid barriers spin with a bound and report a timeout instead of hanging.
-//    Once the trailing matrix fits the SMs' shared memory, eigen_res.cu
+//    columns, each one cooperative kernel (eigen_panel.cu); only the lower
+//    triangle of the trailing matrix is read or updated.  The trailing update
+//    A22 -= V W^T + W V^T runs on the DMMA GEMM as one product with K = 2 NB
+//    ([V W] [W V]^T), over the tiles on or below the diagonal (LAPACK dsyr2k
+//    'L').  Once the trailing matrix fits the SMs' shared memory, eigen_res.cu
 //    factorises the rest.
 // 2. Divide and conquer (LAPACK dstedc / dlaed0-4 structure).  Leaves of at
 //    most 32 rows are diagonalised by a cyclic Jacobi sweep in one CTA each.
@@ -52,16 +38,7 @@ namespace imcom {
 
 namespace {
 
-constexpr int NB = 32;            // tridiagonalisation panel width
-constexpr int TRD_THREADS = 256;  // threads per CTA of the panel kernel
-constexpr int TRD_SLOTS = 3;      // tiles staged per warp (two in flight ahead)
-constexpr int CW = 16;            // columns per symv tile
-constexpr int TR = 64;            // rows per symv tile (two per lane)
-constexpr int CPB = TR / CW;      // column chunks per row block along the diagonal
-// one staging slot: a CW x TR tile, then the TR rows and CW columns of the
-// reflector column it multiplies
-constexpr int TRD_SLOT = CW * TR + TR + CW;
-constexpr size_t TRD_SMEM = (size_t)(TRD_THREADS / 32) * TRD_SLOTS * TRD_SLOT * sizeof(double);
+constexpr int NB = TRD_NB;        // tridiagonalisation panel width
 constexpr int LEAF = 32;          // largest leaf of the divide-and-conquer tree
 constexpr int NBB = 128;          // reflectors per back-transformation block
 constexpr double EPS = 1.1102230246251565e-16;
@@ -73,532 +50,13 @@ __device__ __forceinline__ double warp_sum(double v) {
   return v;
 }
 
-// 16-byte global -> shared copy; bytes < 16 zero-fill the rest (0: all zero)
-__device__ __forceinline__ void cp_async16(double* dst, const double* src, int bytes) {
-  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(src), "r"(bytes)
-               : "memory");
-}
-__device__ __forceinline__ void cp_async8(double* dst, const double* src, int bytes) {
-  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(d), "l"(src), "r"(bytes)
-               : "memory");
-}
-__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-__device__ __forceinline__ void cp_wait_2() { asm volatile("cp.async.wait_group 2;\n" ::: "memory"); }
-__device__ __forceinline__ void cp_wait_0() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
-
-__device__ __forceinline__ double ld_cg(const double* p) {
-  double v;
-  asm volatile("ld.global.cg.f64 %0, [%1];" : "=d"(v) : "l"(p));
-  return v;
-}
-
 // ---------------------------------------------------------------------------
-// Bounded grid barrier (cooperative launch guarantees co-residency).
-// ---------------------------------------------------------------------------
-struct GridSync {
-  unsigned count;  // arrivals so far (monotonic; one barrier = gridDim.x arrivals)
-  unsigned pad0;
-  int err;
-  int pad1;
-};
-
-// Arrive with a release add, wait with acquire loads until every CTA of this
-// barrier generation has arrived.  The wait gives up after `limit` polls and
-// sets the error word instead of spinning forever.  `extra` > 0 (a test of
-// that bound) waits for arrivals that never come.
-__device__ __forceinline__ bool grid_barrier(GridSync* s, long long limit, int extra = 0) {
-  __shared__ int s_ok;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    const unsigned nb = gridDim.x;
-    unsigned old;
-    asm volatile("atom.add.release.gpu.u32 %0, [%1], 1;" : "=r"(old) : "l"(&s->count) : "memory");
-    const unsigned target = (old / nb + 1) * nb + (unsigned)extra;
-    int ok = 1;
-    long long it = 0;
-    while (true) {
-      unsigned cur;
-      asm volatile("ld.acquire.gpu.u32 %0, [%1];" : "=r"(cur) : "l"(&s->count) : "memory");
-      if ((int)(cur - target) >= 0) break;
-      if ((++it & 31) == 0) {
-        if (*(volatile int*)&s->err) {
-          ok = 0;
-          break;
-        }
-        if (it > limit) {
-          atomicExch(&s->err, 1);
-          ok = 0;
-          break;
-        }
-      }
-    }
-    s_ok = ok;
-  }
-  __syncthreads();
-  return s_ok != 0;
-}
-
-// ---------------------------------------------------------------------------
-// 1. Tridiagonalisation
-// ---------------------------------------------------------------------------
-struct TrdAcc {
-  double SW[NB];  // sum_{r >= j+2} A(r, j) W(r, p) for the column j this parity serves
-  double SV[NB];  // sum_{r >= j+2} A(r, j) V(r, p)
-  double vty0;    // x^T A22 x of the raw column x = A(j+1:n, j)
-  double nrm;     // squared norm of the column below its subdiagonal
-};
-
-struct TrdArgs {
-  double* A;
-  long long lda;
-  double* V;  // n x n: column j holds v_j (zero above row j+1, 1 at row j+1)
-  long long ldv;
-  double* W;  // n x NB panel
-  long long ldw;
-  double *d, *e, *tau;
-  double* ypart;  // [chunk][ldy]: row sums of the tiles of one column chunk
-  double* ycol;   // [row block][ldy]: column sums of the tiles of one row block
-  long long ldy;
-  TrdAcc* acc;  // [2] by column parity
-  GridSync* sync;
-  int n, k, b;
-  long long spin;
-  int stall;  // test of the bounded barrier: the first barrier never completes
-};
-
-template <bool CACHED>
-__global__ void __launch_bounds__(TRD_THREADS, 1) trd_panel_kernel(TrdArgs a) {
-  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  constexpr int WPB = TRD_THREADS / 32;
-  constexpr int HP = (NB + WPB - 1) / WPB;  // panel columns per warp in phase B
-  const long long gw = (long long)blockIdx.x * WPB + wib;
-  const long long GW = (long long)gridDim.x * WPB;
-  const int n = a.n, k = a.k;
-  double* A = a.A;
-  const long long lda = a.lda, ldv = a.ldv, ldw = a.ldw;
-  __shared__ double s_pq[2 * NB];            // p = W^T v, q = V^T v of the current column
-  __shared__ double s_rowV[NB], s_rowW[NB];  // row j+1 of V and W
-  __shared__ double s_alpha2;                  // -1/2 tau^2 v^T y of the current column
-  __shared__ double sm_y[WPB][32], sm_c[WPB][32], sm_u[WPB][32];
-  extern __shared__ __align__(16) double trd_tiles[];  // [warp][slot][TRD_SLOT]
-  double* wbuf = trd_tiles + (size_t)wib * TRD_SLOTS * TRD_SLOT;
-  if (*(volatile int*)&a.sync->err) return;  // an earlier panel failed
-
-  // Column k: d(k) and the norm of A(k+2:n, k) (one atomic per CTA).
-  {
-    double part = 0.0;
-    for (long long r0 = k + 2 + gw * 32; r0 < n; r0 += GW * 32) {
-      long long r = r0 + lane;
-      double v = (r < n) ? A[r + k * lda] : 0.0;
-      part += v * v;
-    }
-    part = warp_sum(part);
-    if (lane == 0) sm_y[wib][0] = part;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      double s = 0.0;
-      for (int w = 0; w < WPB; ++w) s += sm_y[w][0];
-      if (s != 0.0) atomicAdd(&a.acc[0].nrm, s);
-    }
-  }
-  if (blockIdx.x == 0 && threadIdx.x == 0) a.d[k] = A[k + k * lda];
-  if (!grid_barrier(a.sync, a.spin, a.stall)) return;
-
-  for (int i = 0; i < a.b; ++i) {
-    const int j = k + i;
-    const int par = i & 1;
-    TrdAcc* cur = a.acc + par;
-    TrdAcc* nxt = a.acc + (par ^ 1);
-    // The tiles cover the trailing matrix of column jg: this column, or for
-    // the cached variant the panel's first column k, so that every warp
-    // keeps the same tiles (in its shared-memory slots) through the panel
-    // and only x changes; x is zero left of and above column j+1 there, and
-    // the chunks wholly left of it (ch < chf) are skipped.
-    const long long jg = CACHED ? k : j;
-    const long long chf = (j - jg) / CW;
-    // rows handled in pairs from an even base row so the loads are 16-byte
-    const long long rbase = (jg + 1) & ~1LL;
-    const long long R = n - (jg + 1);
-    const long long RB = (n - rbase + TR - 1) / TR, NC = (R + CW - 1) / CW;
-    // Tiles on or below the diagonal: row block rb (TR rows from rbase +
-    // TR rb) with column chunks ch < min(NC, CPB (rb + 1)), counted row block
-    // by row block; rb < rbc has CPB (rb + 1) chunks, the rest NC.
-    const long long rbc = min(RB, max(0LL, (NC - 1) / CPB));
-    const long long tri = (long long)CPB * rbc * (rbc + 1) / 2;
-    const long long ntiles = tri + (RB - rbc) * NC;
-
-    // tiles are staged through a TRD_SLOTS-slot shared-memory buffer per warp
-    // by cp.async (zero-filled outside the triangle and below row n), together
-    // with the segments of column j they multiply, so the next two tiles are
-    // in flight while this one is summed
-    const double* colj = A + (long long)j * lda;
-    // tile counts stay far below 2^31 (n^2 / 2048), so 32-bit arithmetic; the
-    // float square root is only a first guess that the loops correct
-    auto decode = [&](int tile, int& rb, int& ch) {
-      if (tile < (int)tri) {
-        // largest rb with CPB rb (rb + 1) / 2 <= tile
-        int q = (int)((sqrtf(1.0f + 8.0f * (float)tile / CPB) - 1.0f) * 0.5f);
-        while (CPB * (q + 1) * (q + 2) / 2 <= tile) ++q;
-        while (q > 0 && CPB * q * (q + 1) / 2 > tile) --q;
-        rb = q;
-        ch = tile - CPB * q * (q + 1) / 2;
-      } else {
-        const unsigned t2 = (unsigned)(tile - (int)tri), nc = (unsigned)NC;
-        const unsigned qq = t2 / nc;
-        rb = (int)rbc + (int)qq;
-        ch = (int)(t2 - qq * nc);
-      }
-    };
-    // x's segments for tile (rb, ch): rows r, r + 1 and columns c0 ..
-    auto issue_x = [&](int rb, int ch, int slot) {
-      const long long r = rbase + (long long)rb * TR + 2 * lane;
-      const long long c0 = jg + 1 + (long long)ch * CW, c1 = min((long long)n, c0 + CW);
-      double* dst = wbuf + slot * TRD_SLOT + 2 * lane;
-      const bool okr = r < n;
-      cp_async16(dst + CW * TR, okr ? colj + r : A, okr ? (r + 1 < n ? 16 : 8) : 0);
-      if (lane < CW) {
-        const bool okc = c0 + lane < c1;
-        cp_async8(wbuf + slot * TRD_SLOT + CW * TR + TR + lane, okc ? colj + c0 + lane : A,
-                  okc ? 8 : 0);
-      }
-    };
-    auto issue = [&](int rb, int ch, int slot) {
-      const long long r = rbase + (long long)rb * TR + 2 * lane;
-      const long long c0 = jg + 1 + (long long)ch * CW, c1 = min((long long)n, c0 + CW);
-      double* dst = wbuf + slot * TRD_SLOT + 2 * lane;
-#pragma unroll
-      for (int u = 0; u < CW; ++u) {
-        const long long c = c0 + u;
-        // a row of the pair on or below the diagonal; the second row only
-        // if it exists
-        const bool ok = c < c1 && r + 1 >= c && r < n;
-        cp_async16(dst + u * TR, ok ? A + r + c * lda : A, ok ? (r + 1 < n ? 16 : 8) : 0);
-      }
-      const bool okr = r < n;
-      cp_async16(dst + CW * TR, okr ? colj + r : A, okr ? (r + 1 < n ? 16 : 8) : 0);
-      if (lane < CW) {
-        const bool okc = c0 + lane < c1;
-        cp_async8(wbuf + slot * TRD_SLOT + CW * TR + TR + lane, okc ? colj + c0 + lane : A,
-                  okc ? 8 : 0);
-      }
-    };
-    // Phase A forms A22 x for the raw column x = A(j+1:n, j); the reflector
-    // v = scl x + delta e_{j+1} (delta = 1 - scl x(j+1)) only enters in
-    // phase B, y0 = A22 v = scl (A22 x) + delta A22(:, j+1), so the tiles do
-    // not wait for the reflector.  Its loads are issued now, used after the
-    // tile loop.
-    // decoded indices of this warp's next two tiles
-    int rb_n = 0, ch_n = 0, rb_m = 0, ch_m = 0;
-    if constexpr (CACHED) {
-      // the warp's tiles (at most TRD_SLOTS) sit in slots 0, 1, .. for the
-      // whole panel: the first column loads them, every column its x
-      int q = 0;
-      for (long long tile = gw; tile < ntiles; tile += GW, ++q) {
-        int rb, ch;
-        decode((int)tile, rb, ch);
-        if (i == 0) issue(rb, ch, q);
-        else issue_x(rb, ch, q);
-      }
-      cp_commit();
-    } else {
-      if (gw < ntiles) {
-        decode((int)gw, rb_n, ch_n);
-        issue(rb_n, ch_n, 0);
-      }
-      cp_commit();
-      if (gw + GW < ntiles) {
-        decode((int)(gw + GW), rb_m, ch_m);
-        issue(rb_m, ch_m, 1);
-      }
-      cp_commit();
-    }
-    const double alpha = ld_cg(A + (j + 1) + (long long)j * lda);
-    const double xn2 = ld_cg(&cur->nrm);
-    // A(j+1, j+1) before this column's phase B rewrites column j+1
-    const double a11 = (wib == 0) ? ld_cg(A + (j + 1) + (long long)(j + 1) * lda) : 0.0;
-    if (blockIdx.x == 0 && threadIdx.x < 2 * NB + 2) {
-      // clear the other parity's accumulators (last read one phase ago)
-      if (threadIdx.x < NB) nxt->SW[threadIdx.x] = 0.0;
-      else if (threadIdx.x < 2 * NB) nxt->SV[threadIdx.x - NB] = 0.0;
-      else if (threadIdx.x == 2 * NB) nxt->vty0 = 0.0;
-      else nxt->nrm = 0.0;
-    }
-    // Row j+1 of V and W, and p = W^T v = W(j+1, :) + scl * SW, q = V^T v
-    // likewise (sums from the previous column's phase B); loaded now, kept
-    // in shared memory for phase B after the tile loop
-    double wr1 = 0.0, vr1 = 0.0, sw1 = 0.0, sv1 = 0.0;
-    if (wib == 0 && lane < i) {
-      wr1 = ld_cg(a.W + (j + 1) + lane * ldw);
-      vr1 = ld_cg(a.V + (j + 1) + (k + lane) * ldv);
-      sw1 = ld_cg(&cur->SW[lane]);
-      sv1 = ld_cg(&cur->SV[lane]);
-    }
-    // ---- phase A: A22 x from the lower triangle (LAPACK dsymv 'L').
-    // Tile (rb, ch) reads A(r, c) for r >= c once and gives the row sums
-    // sum_c A(r, c) x(c) (to ypart[ch]) and the column sums
-    // sum_{r > c} A(r, c) x(r) (to ycol[rb]); (A22 x)(r) is the sum of both
-    // kinds.  x^T A22 x is summed per warp, then per CTA, and added with one
-    // atomic per CTA. ----
-    double vty_part = 0.0;
-    // Tile (rb, ch) in `slot`: row sums to ypart[ch], column sums to
-    // ycol[rb], its share of x^T A22 x to vty_part.
-    auto sum_tile = [&](int rb, int ch, int slot) {
-      const long long r = rbase + (long long)rb * TR + 2 * lane;
-      const long long c0 = jg + 1 + (long long)ch * CW, c1 = min((long long)n, c0 + CW);
-      const double* sl = wbuf + slot * TRD_SLOT;
-      const double2 vraw = reinterpret_cast<const double2*>(sl + CW * TR)[lane];
-      // raw column-j values at rows r, r + 1 and at columns c0 .. c0 + CW - 1
-      // (zero-filled past row n); rows at or above j lie above x (only row j
-      // when rbase = j; the cached tiles' columns at or left of j are zeroed
-      // before the tile is summed)
-      const double* vcol = sl + CW * TR + TR;
-      const double v0 = (r <= j) ? 0.0 : vraw.x, v1 = (r + 1 <= j) ? 0.0 : vraw.y;
-      const double2* av = reinterpret_cast<const double2*>(sl) + lane;
-      const int dr = (int)(r - c0);  // this lane's first row relative to column c0
-      double acc0 = 0.0, acc1 = 0.0, vtz = 0.0;
-      // two halves of CW / 2 columns: row sums, then the column sums of the
-      // half transpose-reduced over the warp (lane L ends with the sum for
-      // column c0 + H + (L >> 2)), so only CW / 2 partials are live at once.
-      // Tiles crossing the diagonal mask A(r, c) with r < c from the row sums
-      // and r <= c from the column sums; the others need no mask.
-      auto tile_sums = [&](auto masked) {
-#pragma unroll
-        for (int H = 0; H < CW; H += CW / 2) {
-          double z[CW / 2];
-#pragma unroll
-          for (int u = 0; u < CW / 2; ++u) {
-            const int cu = H + u;
-            const double2 e2 = av[cu * (TR / 2)];
-            const double vc = vcol[cu];
-            double ax = e2.x, zx = e2.x, zy = e2.y;
-            if (decltype(masked)::value) {
-              ax = (dr >= cu) ? e2.x : 0.0;
-              zx = (dr > cu) ? e2.x : 0.0;
-              zy = (dr + 1 > cu) ? e2.y : 0.0;
-            }
-            acc0 = fma(ax, vc, acc0);
-            acc1 = fma(e2.y, vc, acc1);
-            z[u] = fma(zy, v1, zx * v0);
-          }
-#pragma unroll
-          for (int h = CW / 4, m = 16; h >= 1; h >>= 1, m >>= 1) {
-            const bool hi = (lane & m) != 0;
-#pragma unroll
-            for (int q = 0; q < h; ++q) {
-              const double send = hi ? z[q] : z[q + h];
-              const double keep = hi ? z[q + h] : z[q];
-              z[q] = keep + __shfl_xor_sync(0xffffffffu, send, m);
-            }
-          }
-          double zc = z[0] + __shfl_xor_sync(0xffffffffu, z[0], 2);
-          zc += __shfl_xor_sync(0xffffffffu, zc, 1);
-          const long long cz = c0 + H + (lane >> 2);
-          if (!(lane & 3) && cz < c1) {
-            a.ycol[(long long)rb * a.ldy + cz] = zc;
-            vtz += vcol[H + (lane >> 2)] * zc;
-          }
-        }
-      };
-      if (rbase + (long long)rb * TR <= c0 + CW - 1) tile_sums(std::true_type{});
-      else tile_sums(std::false_type{});
-      if (r >= j + 1 && r < n) a.ypart[(long long)ch * a.ldy + r] = acc0;
-      if (r + 1 >= j + 1 && r + 1 < n) a.ypart[(long long)ch * a.ldy + r + 1] = acc1;
-      vty_part += v0 * acc0 + v1 * acc1 + vtz;
-    };
-    if constexpr (CACHED) {
-      cp_wait_0();
-      __syncwarp();
-      int q = 0;
-      for (long long tile = gw; tile < ntiles; tile += GW, ++q) {
-        int rb, ch;
-        decode((int)tile, rb, ch);
-        if (ch < chf) continue;  // every column left of j+1: x is zero
-        const long long c0 = jg + 1 + (long long)ch * CW;
-        double* vc = wbuf + q * TRD_SLOT + CW * TR + TR;
-        if (lane < CW && c0 + lane <= j) vc[lane] = 0.0;
-        __syncwarp();
-        sum_tile(rb, ch, q);
-      }
-    } else {
-      int slot = 0;
-      for (long long tile = gw; tile < ntiles; tile += GW, slot = (slot + 1) % TRD_SLOTS) {
-        const int rb = rb_n, ch = ch_n;
-        rb_n = rb_m;
-        ch_n = ch_m;
-        if (tile + 2 * GW < ntiles) {
-          decode((int)(tile + 2 * GW), rb_m, ch_m);
-          issue(rb_m, ch_m, (slot + 2) % TRD_SLOTS);
-        }
-        cp_commit();
-        cp_wait_2();
-        sum_tile(rb, ch, slot);
-      }
-    }
-    cp_wait_0();
-    // Householder reflector of x = A(j+1:n, j) (LAPACK dlarfg)
-    double beta, t, scl;
-    if (xn2 == 0.0) {
-      t = 0.0;
-      beta = alpha;
-      scl = 0.0;
-    } else {
-      beta = -copysign(sqrt(alpha * alpha + xn2), alpha);
-      t = (beta - alpha) / beta;
-      scl = 1.0 / (alpha - beta);
-    }
-    const double delta = 1.0 - scl * alpha;
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-      a.e[j] = beta;
-      a.tau[j] = t;
-    }
-    if (wib == 0 && lane < i) {
-      s_rowW[lane] = wr1;
-      s_rowV[lane] = vr1;
-      s_pq[lane] = wr1 + scl * sw1;
-      s_pq[NB + lane] = vr1 + scl * sv1;
-    }
-    vty_part = warp_sum(vty_part);
-    if (lane == 0) sm_u[wib][0] = vty_part;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      double s = 0.0;
-      for (int w = 0; w < WPB; ++w) s += sm_u[w][0];
-      if (s != 0.0) atomicAdd(&cur->vty0, s);
-    }
-    if (!grid_barrier(a.sync, a.spin)) return;
-
-    // ---- phase B: w, the next column, its norm and dot products ----
-    const bool next = (i + 1 < a.b);
-    bool have_w1 = false;
-    // one 32-row block per CTA at a time; the warps split the chunk partials
-    // and the panel columns, then reduce through shared memory
-    // warp 0: this lane's share of y0(j+1), loaded alongside the first row
-    // block's partial sums
-    double y1 = 0.0;
-    if (wib == 0) {
-      if (lane >= chf && lane < min(NC, (long long)CPB))
-        y1 = __ldcg(a.ypart + lane * a.ldy + (j + 1));
-      for (long long q = lane; q < RB; q += 32) y1 += __ldcg(a.ycol + q * a.ldy + (j + 1));
-    }
-    for (long long rb = blockIdx.x; j + 1 + rb * 32 < n; rb += gridDim.x) {
-      const long long r = j + 1 + rb * 32 + lane;
-      const bool valid = r < n;
-      // issue every load of the row block first
-      double ys = 0.0, vp[HP] = {}, wp[HP] = {};
-      double vr = 0.0, aold = 0.0;
-      const double vty0 = __ldcg(&cur->vty0);
-      if (valid) {
-        // row sums of the chunks its row block covers, column sums of the
-        // row blocks below its chunk
-        const long long ncr = min(NC, (long long)CPB * ((r - rbase) / TR + 1));
-        const long long rb0 = (r - (jg + 1)) / CW / CPB;
-#pragma unroll 4
-        for (long long ch = chf + wib; ch < ncr; ch += WPB) ys += __ldcg(a.ypart + ch * a.ldy + r);
-#pragma unroll 4
-        for (long long q = rb0 + wib; q < RB; q += WPB) ys += __ldcg(a.ycol + q * a.ldy + r);
-#pragma unroll
-        for (int h = 0; h < HP; ++h) {
-          const int p = wib + WPB * h;
-          if (p < i) {
-            vp[h] = __ldcg(a.V + r + (k + p) * ldv);
-            wp[h] = __ldcg(a.W + r + p * ldw);
-          }
-        }
-        vr = (r == j + 1) ? 1.0 : __ldcg(colj + r) * scl;
-        aold = __ldcg(A + r + (long long)(j + 1) * lda);
-      }
-      if (!have_w1 && wib == 0) {
-        // v^T y0 = scl^2 x^T A22 x + 2 scl delta (A22 x)(j+1) + delta^2 A(j+1, j+1),
-        // alpha2 = -1/2 tau^2 v^T y with v^T y = v^T y0 - 2 (V^T v).(W^T v), and
-        // w(j+1) (the new entry of row j+1 of W)
-        const double s1 = warp_sum(y1);
-        double qp = 0.0;
-        for (int p = 0; p < i; ++p) qp += s_pq[NB + p] * s_pq[p];
-        const double vty = scl * scl * vty0 + 2.0 * scl * delta * s1 + delta * delta * a11;
-        const double al2 = -0.5 * t * t * (vty - 2.0 * qp);
-        double corr = (lane < i) ? s_rowV[lane] * s_pq[lane] + s_rowW[lane] * s_pq[NB + lane] : 0.0;
-        corr = warp_sum(corr);
-        if (lane == 0) {
-          s_alpha2 = al2;
-          if (next) {
-            s_rowW[i] = t * ((scl * s1 + delta * a11) - corr) + al2;
-            s_rowV[i] = 1.0;
-          }
-        }
-      }
-      have_w1 = true;
-      double cs = 0.0, us = 0.0;
-#pragma unroll
-      for (int h = 0; h < HP; ++h) {
-        const int p = wib + WPB * h;
-        if (p < i) {
-          cs += vp[h] * s_pq[p] + wp[h] * s_pq[NB + p];
-          us += vp[h] * s_rowW[p] + wp[h] * s_rowV[p];
-        }
-      }
-      sm_y[wib][lane] = ys;
-      sm_c[wib][lane] = cs;
-      sm_u[wib][lane] = us;
-      __syncthreads();
-      double y0 = 0.0, corr = 0.0, upd = 0.0;
-#pragma unroll
-      for (int w = 0; w < WPB; ++w) {
-        y0 += sm_y[w][lane];
-        corr += sm_c[w][lane];
-        upd += sm_u[w][lane];
-      }
-      y0 = scl * y0 + delta * aold;  // A22 v from A22 x
-      const double wr = t * (y0 - corr) + s_alpha2 * vr;
-      if (valid && wib == 0) {
-        a.V[r + (long long)j * ldv] = vr;
-        a.W[r + i * ldw] = wr;
-      }
-      if (next) {
-        double anew = 0.0;
-        if (valid) {
-          upd += vr * s_rowW[i] + wr * s_rowV[i];
-          anew = aold - upd;
-          if (wib == 0) {
-            A[r + (long long)(j + 1) * lda] = anew;
-            if (r == j + 1) a.d[j + 1] = anew;
-          }
-        }
-        // column j+1's dot products with W, V over rows >= j+3 and its norm
-        const double am = (valid && r >= j + 3) ? anew : 0.0;
-#pragma unroll
-        for (int h = 0; h < HP; ++h) {
-          const int p = wib + WPB * h;
-          if (p <= i) {
-            const double wv = (p == i) ? wr : wp[h];
-            const double vv = (p == i) ? vr : vp[h];
-            const double sw = warp_sum(am * wv), sv = warp_sum(am * vv);
-            if (lane == 0) {
-              atomicAdd(&nxt->SW[p], sw);
-              atomicAdd(&nxt->SV[p], sv);
-            }
-          }
-        }
-        if (wib == 0) {
-          const double nr = warp_sum(am * am);
-          if (lane == 0) atomicAdd(&nxt->nrm, nr);
-        }
-      }
-      __syncthreads();
-    }
-    if (!grid_barrier(a.sync, a.spin)) return;
-  }
-
-}
-
-// ---------------------------------------------------------------------------
-// 1b. The last columns of the tridiagonalisation in one thread-block cluster
-// (where IMCOM_OPT_TAIL_CTAS asks for one; by default eigen_res.cu takes over).
+// 1. The last columns of the tridiagonalisation in one thread-block cluster
+// (where IMCOM_OPT_TAIL_CTAS asks for one or the context has fewer than 8 SMs; else
+// eigen_res.cu takes over).
 //
 // Once the trailing matrix is small, every column of the panel kernel is a
-// chain of dependent L2 round trips and two grid barriers (~9 us whatever
-// the size).  From trailing size S <= tail_max the rest of the matrix is
+// chain of dependent exchanges through L2 (~8 us whatever the size).  From trailing size S <= tail_max the rest of the matrix is
 // factorised by one cluster of up to 16 CTAs holding it in distributed
 // shared memory: full symmetric rows, CTA q owning rows [q rpc, (q+1) rpc).
 // Unblocked LAPACK dsytd2 'L', per column j:
@@ -1526,25 +984,24 @@ static void tail_config(imcom_ctx* ctx, int* tail_ctas_out, int* tail_max_out) {
 
 // The launch sequence of the tridiagonalisation: panels, their trailing
 // updates and the cluster tail.  `capturing`: recorded into a graph, so the
-// periodic host check of the barrier's error word is left to the caller.
+// periodic host check of the exchanges' error word is left to the caller.
 static int sytrd_launches(imcom_ctx* ctx, DMat& Aw, DMat& Vall, double* d, double* e,
-                          double* tau, double* W, long long ldw, double* ypart, double* ycol,
-                          long long ldy, void* accbuf, long long spin, double* XY, int tail_ctas,
-                          int tail_max, int res_max, void* resbuf, bool capturing) {
+                          double* tau, double* W, long long ldw, int* err, void* panbuf,
+                          long long spin, double* XY, int tail_ctas, int tail_max, int res_max,
+                          void* resbuf, bool capturing) {
   const int n = (int)Aw.rows;
-  int grid = sm_count(ctx);  // one CTA per SM: the cheapest grid barrier
-  TrdAcc* acc = (TrdAcc*)accbuf;
-  GridSync* sync = (GridSync*)((char*)accbuf + 2 * sizeof(TrdAcc) + 64);
-  int* flag = &sync->err;
-  IMC_CUDA(cudaMemsetAsync(sync, 0, sizeof(GridSync), ctx->stream));
+  const int grid = sm_count(ctx);  // one CTA per SM
+  const int stall = (ctx->stall_test & IMCOM_STALL_TRIDIAG) ? 1 : 0;
+  IMC_CUDA(cudaMemsetAsync(err, 0, sizeof(int), ctx->stream));
+  // tags of an earlier call
+  if (panbuf) IMC_CUDA(cudaMemsetAsync(panbuf, 0, panel_bytes(n, panel_grid(ctx, n)), ctx->stream));
   bool tail_done = false;
   for (int k = 0; k < n - 1; k += NB) {
     // the trailing matrix fits the SMs' shared memory: 3.7 us per column from
-    // 2048 down (2.0 us from 500), against 11 to 8 us on panels and 7.2 us in
+    // 2048 down (2.0 us from 500), against 11 to 7.4 us on panels and 7.2 us in
     // the cluster tail below
     if (n - k <= res_max) {
-      IMC_TRY(resident_tridiag(ctx, Aw, Vall, d, e, tau, k, grid, resbuf, flag, spin,
-                               (ctx->stall_test & IMCOM_STALL_TRIDIAG) ? 1 : 0));
+      IMC_TRY(resident_tridiag(ctx, Aw, Vall, d, e, tau, k, grid, resbuf, err, spin, stall));
       tail_done = true;
       break;
     }
@@ -1569,23 +1026,8 @@ static int sytrd_launches(imcom_ctx* ctx, DMat& Aw, DMat& Vall, double* d, doubl
       break;
     }
     const int b = std::min(NB, n - 1 - k);
-    IMC_CUDA(cudaMemsetAsync(accbuf, 0, 2 * sizeof(TrdAcc), ctx->stream));
-    static_assert(2 * sizeof(TrdAcc) + 64 + sizeof(GridSync) <= 4096, "panel scratch");
-    TrdArgs a{Aw.p, Aw.ld, Vall.p, Vall.ld, W, ldw, d, e, tau, ypart, ycol, ldy, acc, sync, n,
-              k, b, spin, (ctx->stall_test & IMCOM_STALL_TRIDIAG) ? 1 : 0};
-    void* args[] = {&a};
-    // Tiles of the panel's first trailing matrix: when every warp has at
-    // most TRD_SLOTS of them, they stay in shared memory for the panel's
-    // columns (read from L2 once per panel instead of once per column).
-    const long long rbase = (k + 1) & ~1LL, R = n - (k + 1);
-    const long long RB = (n - rbase + TR - 1) / TR, NC = (R + CW - 1) / CW;
-    const long long rbc = std::min(RB, std::max(0LL, (NC - 1) / CPB));
-    const long long ntiles = (long long)CPB * rbc * (rbc + 1) / 2 + (RB - rbc) * NC;
-    const bool cached = ntiles <= (long long)TRD_SLOTS * grid * (TRD_THREADS / 32);
-    IMC_CUDA(cudaLaunchCooperativeKernel(
-        cached ? (void*)trd_panel_kernel<true> : (void*)trd_panel_kernel<false>, grid,
-        TRD_THREADS, args, TRD_SMEM, ctx->stream));
-    IMC_LAUNCH();
+    IMC_TRY(panel_launch(ctx, Aw, Vall, W, ldw, d, e, tau, k, b, panel_grid(ctx, n), panbuf, err, spin,
+                         stall));
     const int t0 = k + b, rem = n - t0;
     if (rem > 0) {
       // A22 -= V W^T + W V^T as one K = 2b product over the lower triangle
@@ -1600,10 +1042,10 @@ static int sytrd_launches(imcom_ctx* ctx, DMat& Aw, DMat& Vall, double* d, doubl
       IMC_TRY(dgemm_lower_nt(ctx, rem, 2 * b, -1.0, X + t0, ldx, Y + t0, ldx, 1.0,
                              Aw.p + t0 + (long long)t0 * Aw.ld, Aw.ld));
     }
-    // a timed-out barrier ends the factorisation with an error
+    // a timed-out exchange ends the factorisation with an error
     if (!capturing && (k / NB) % 16 == 15) {
       int h = 0;
-      IMC_CUDA(cudaMemcpyAsync(&h, flag, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+      IMC_CUDA(cudaMemcpyAsync(&h, err, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
       IMC_CUDA(cudaStreamSynchronize(ctx->stream));
       if (h) return set_err(ctx, IMCOM_ERR_EIGEN, "tridiagonalisation grid barrier timed out");
     }
@@ -1622,35 +1064,22 @@ static int sytrd_launches(imcom_ctx* ctx, DMat& Aw, DMat& Vall, double* d, doubl
 // it, later calls launch the graph.  A capture the driver refuses leaves the
 // direct path in place.
 static int sytrd_gpu(imcom_ctx* ctx, DMat& Aw, DMat& Vall, double* d, double* e, double* tau,
-                     double* W, long long ldw, double* ypart, double* ycol, long long ldy,
-                     void* accbuf, long long spin, double* XY, void* resbuf) {
+                     double* W, long long ldw, int* err, void* panbuf, long long spin, double* XY,
+                     int res_max, void* resbuf) {
   const int n = (int)Aw.rows;
   int dev = ctx->device, coop = 0;
   cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
   if (!coop) return set_err(ctx, IMCOM_ERR_CUDA, "device lacks cooperative launch");
-  int per_sm = 0, per_sm_c = 0;
-  IMC_CUDA(cudaFuncSetAttribute(trd_panel_kernel<false>,
-                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TRD_SMEM));
-  IMC_CUDA(cudaFuncSetAttribute(trd_panel_kernel<true>,
-                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TRD_SMEM));
-  IMC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, trd_panel_kernel<false>,
-                                                         TRD_THREADS, TRD_SMEM));
-  IMC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_c, trd_panel_kernel<true>,
-                                                         TRD_THREADS, TRD_SMEM));
-  if (per_sm < 1 || per_sm_c < 1)
-    return set_err(ctx, IMCOM_ERR_CUDA, "panel kernel does not fit on an SM");
+  if (panbuf) IMC_TRY(panel_prepare(ctx));
   int tail_ctas = 0, tail_max = 0;
-  const int res_max = ctx->tail_ctas == 0 ? resident_max(ctx, sm_count(ctx)) : 0;
   if (!res_max) tail_config(ctx, &tail_ctas, &tail_max);
-  GridSync* sync = (GridSync*)((char*)accbuf + 2 * sizeof(TrdAcc) + 64);
   EigWork* ew = eig_work(ctx);
   const long long key[] = {n, (long long)(uintptr_t)Aw.p, Aw.ld, (long long)(uintptr_t)Vall.p,
                            Vall.ld, (long long)(uintptr_t)d, (long long)(uintptr_t)e,
                            (long long)(uintptr_t)tau, (long long)(uintptr_t)W, ldw,
-                           (long long)(uintptr_t)ypart, (long long)(uintptr_t)ycol, ldy,
-                           (long long)(uintptr_t)accbuf, spin, (long long)(uintptr_t)XY,
-                           sm_count(ctx), tail_ctas, tail_max, ctx->stall_test, res_max,
-                           (long long)(uintptr_t)resbuf};
+                           (long long)(uintptr_t)err, (long long)(uintptr_t)panbuf, spin,
+                           (long long)(uintptr_t)XY, sm_count(ctx), tail_ctas, tail_max,
+                           ctx->stall_test, res_max, (long long)(uintptr_t)resbuf};
   constexpr int NKEY = (int)(sizeof(key) / sizeof(key[0]));
   static_assert(NKEY <= EigWork::kTrdKey, "graph key size");
   const bool same = std::equal(key, key + NKEY, ew->trd_key);
@@ -1673,8 +1102,8 @@ static int sytrd_gpu(imcom_ctx* ctx, DMat& Aw, DMat& Vall, double* d, double* e,
       ok = cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeRelaxed) == cudaSuccess;
       int st = 0;
       if (ok) {
-        st = sytrd_launches(ctx, Aw, Vall, d, e, tau, W, ldw, ypart, ycol, ldy, accbuf, spin,
-                            XY, tail_ctas, tail_max, res_max, resbuf, true);
+        st = sytrd_launches(ctx, Aw, Vall, d, e, tau, W, ldw, err, panbuf, spin, XY,
+                            tail_ctas, tail_max, res_max, resbuf, true);
         ok = cudaStreamEndCapture(ctx->stream, &graph) == cudaSuccess && st == 0 && graph;
       }
     }
@@ -1689,16 +1118,16 @@ static int sytrd_gpu(imcom_ctx* ctx, DMat& Aw, DMat& Vall, double* d, double* e,
     } else {
       ew->trd_graph_off = true;  // run directly from now on
       ctx->err.clear();
-      IMC_TRY(sytrd_launches(ctx, Aw, Vall, d, e, tau, W, ldw, ypart, ycol, ldy, accbuf, spin,
-                             XY, tail_ctas, tail_max, res_max, resbuf, false));
+      IMC_TRY(sytrd_launches(ctx, Aw, Vall, d, e, tau, W, ldw, err, panbuf, spin, XY,
+                            tail_ctas, tail_max, res_max, resbuf, false));
     }
   } else {
-    IMC_TRY(sytrd_launches(ctx, Aw, Vall, d, e, tau, W, ldw, ypart, ycol, ldy, accbuf, spin, XY,
+    IMC_TRY(sytrd_launches(ctx, Aw, Vall, d, e, tau, W, ldw, err, panbuf, spin, XY,
                            tail_ctas, tail_max, res_max, resbuf, false));
   }
-  // a timed-out grid barrier ends the factorisation with an error
+  // a timed-out exchange ends the factorisation with an error
   int h = 0;
-  IMC_CUDA(cudaMemcpyAsync(&h, &sync->err, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+  IMC_CUDA(cudaMemcpyAsync(&h, err, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
   IMC_CUDA(cudaStreamSynchronize(ctx->stream));
   if (h) return set_err(ctx, IMCOM_ERR_EIGEN, "tridiagonalisation grid barrier timed out");
   return 0;
@@ -1723,8 +1152,7 @@ int eigen_dc(imcom_ctx* ctx, const DMat& A, DMat& Wout, double* wout) {
   const long long ld = Wout.ld;
   const size_t nn = (size_t)ld * n;
   // scratch vectors and small matrices in one allocation
-  const long long ldw = pad_ld(n), ldy = pad_ld(n);
-  const long long nch = (n + CW - 1) / CW + 1, nrb = (n + TR - 1) / TR + 1;
+  const long long ldw = pad_ld(n);
   size_t off = 0;
   auto take = [&](size_t bytes) {
     size_t o = off;
@@ -1732,9 +1160,17 @@ int eigen_dc(imcom_ctx* ctx, const DMat& A, DMat& Wout, double* wout) {
     return o;
   };
   size_t o_d = take(n * 8), o_e = take(n * 8), o_tau = take(n * 8), o_dt = take(n * 8);
-  size_t o_W = take((size_t)ldw * NB * 8), o_y = take((size_t)ldy * (nch + nrb) * 8);
+  size_t o_W = take((size_t)ldw * NB * 8);
   size_t o_XY = take((size_t)ldw * 4 * NB * 8);
-  size_t o_acc = take(4096), o_res = take(resident_bytes(n));
+  const bool two = ctx->eig_mode == IMCOM_EIGH_TWOSTAGE;
+  // the trailing size from which the reduction stays in shared memory, and
+  // whether panels run before it.  Shares below 8 SMs keep the cluster tail: n = 400
+  // takes 3.1 ms on 3 SMs' shared memory and 2.1 in the cluster, but 1.4 on 8
+  const int res_max =
+      ctx->tail_ctas == 0 && sm_count(ctx) >= 8 ? resident_max(ctx, sm_count(ctx)) : 0;
+  const bool panels = !two && n > res_max;
+  size_t o_res = take(resident_bytes(n));
+  size_t o_pan = take(panels ? panel_bytes(n, panel_grid(ctx, n)) : 0);
   size_t o_split = take((size_t)n * 4), o_nodes = take((size_t)n * sizeof(Node));
   size_t o_wk = take(((size_t)n * 8 + 16) * 9 + ((size_t)n * 4 + 16) * 8 + ((size_t)n * 24 + 32) +
                      4096);
@@ -1742,8 +1178,7 @@ int eigen_dc(imcom_ctx* ctx, const DMat& A, DMat& Wout, double* wout) {
   const size_t npair_bt = (nblk_bt + 1) / 2;
   size_t o_T = take(npair_bt * 4 * NBB * NBB * 8), o_G = take(npair_bt * 4 * NBB * NBB * 8);
   size_t o_X = take((size_t)2 * NBB * ld * 8 * 2);
-  size_t o_err = take(64);
-  const bool two = ctx->eig_mode == IMCOM_EIGH_TWOSTAGE;
+  size_t o_err = take(64), o_terr = take(64);
   size_t o_2s = take(two ? twostage_bytes(n) : 0);
   IMC_TRY(eig_buf(ctx, off + 256));
   char* base = (char*)ew->buf;
@@ -1752,7 +1187,6 @@ int eigen_dc(imcom_ctx* ctx, const DMat& A, DMat& Wout, double* wout) {
   double* tau = (double*)(base + o_tau);
   double* dt = (double*)(base + o_dt);
   double* Wp = (double*)(base + o_W);
-  double* yp = (double*)(base + o_y);
   int* dsplit = (int*)(base + o_split);
   Node* dnodes = (Node*)(base + o_nodes);
   double* Tb = (double*)(base + o_T);
@@ -1764,14 +1198,18 @@ int eigen_dc(imcom_ctx* ctx, const DMat& A, DMat& Wout, double* wout) {
   // ---- 1. tridiagonalisation ----
   stage_begin(ctx, ST_EIG_TRD);
   IMC_TRY(copy_mat(ctx, A.p, A.ld, Aw.p, Aw.ld, n, n));
+  if (n % 8)  // the panels read rows up to the next multiple of 8
+    IMC_CUDA(cudaMemset2DAsync(Aw.p + n, Aw.ld * sizeof(double), 0, (8 - n % 8) * sizeof(double), n,
+                               ctx->stream));
   IMC_CUDA(cudaMemsetAsync(Vall.p, 0, Vall.bytes(), ctx->stream));
   IMC_CUDA(cudaMemsetAsync(Wp, 0, (size_t)ldw * NB * 8, ctx->stream));
   if (two)
     IMC_TRY(twostage_tridiag(ctx, Aw, Vall, d, e, tau, Wp, ldw, (double*)(base + o_XY),
                              base + o_2s, spin));
   else
-    IMC_TRY(sytrd_gpu(ctx, Aw, Vall, d, e, tau, Wp, ldw, yp, yp + (size_t)ldy * nch, ldy,
-                      base + o_acc, spin, (double*)(base + o_XY), base + o_res));
+    IMC_TRY(sytrd_gpu(ctx, Aw, Vall, d, e, tau, Wp, ldw, (int*)(base + o_terr),
+                      panels ? base + o_pan : nullptr, spin, (double*)(base + o_XY), res_max,
+                      base + o_res));
   stage_end(ctx, ST_EIG_TRD);
   stage_begin(ctx, ST_EIG_DC);
 

@@ -34,6 +34,7 @@
 
 #include "common.cuh"
 #include "eigen.cuh"
+#include "tagged.cuh"
 
 namespace imcom {
 
@@ -61,23 +62,6 @@ struct ResArgs {
   long long spin;
   int stall;  // test of the bounded polls: the first column's values never come
 };
-
-__device__ __forceinline__ void st_tagged(ulonglong2* p, double v, unsigned tag) {
-  asm volatile(
-      "{\n .reg .b128 t;\n mov.b128 t, {%1, %2};\n st.relaxed.gpu.global.b128 [%0], t;\n}\n" ::"l"(p),
-      "l"(__double_as_longlong(v)), "l"((unsigned long long)tag)
-      : "memory");
-}
-
-__device__ __forceinline__ ulonglong2 ld_tagged(const ulonglong2* p) {
-  ulonglong2 r;
-  asm volatile(
-      "{\n .reg .b128 t;\n ld.relaxed.gpu.global.b128 t, [%2];\n mov.b128 {%0, %1}, t;\n}\n"
-      : "=l"(r.x), "=l"(r.y)
-      : "l"(p)
-      : "memory");
-  return r;
-}
 
 __device__ __forceinline__ double wsum(double v) {
 #pragma unroll

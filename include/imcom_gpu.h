@@ -93,7 +93,7 @@ typedef struct imcom_ctx imcom_ctx;
 #define IMCOM_OPT_SM_SHARE 10
 /* How the tridiagonalisation ends: 0 (default) = the trailing matrix resident
  * in the shared memory of this context's SMs (up to order 2048 on 148 SMs),
- * one exchange per column; 8 or 16 = a thread-block cluster of that many
+ * one exchange per column (a share below 8 SMs: the cluster); 8 or 16 = a thread-block cluster of that many
  * CTAs (8 if 16 cannot be placed) once the trailing matrix fits its
  * distributed shared memory; -1 = panels to the end.  A 16-CTA cluster must
  * find 16 free SMs in one GPC, which contexts working side by side can make
@@ -149,10 +149,9 @@ typedef struct imcom_ctx imcom_ctx;
  *    with IMCOM_PREC_SPLIT) issues no copies, so the MMA issuer's first wait
  *    (bounded at 2 s) runs out; the kernel drains, frees its tensor memory
  *    and returns, and the next bisection returns IMCOM_ERR_SPLIT;
- *  IMCOM_STALL_TRIDIAG: the first grid barrier of the tridiagonalisation
- *    waits for one arrival more than the grid makes (or, where no panel runs,
- *    the first exchange of the resident columns for a value that nobody
- *    publishes), so it gives up after IMCOM_OPT_EIGEN_MAXITER polls and
+ *  IMCOM_STALL_TRIDIAG: the first exchange of the tridiagonalisation's
+ *    panels (or, where no panel runs, of the resident columns) waits for a
+ *    value that nobody publishes, so it gives up after IMCOM_OPT_EIGEN_MAXITER polls and
  *    imcom_gpu_eigen_A returns IMCOM_ERR_EIGEN (not in the cluster tail).
  * The context stays usable: clear the option and the next call runs
  * normally. */

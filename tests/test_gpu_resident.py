@@ -44,7 +44,7 @@ def _check(A, Q, L):
 
 @pytest.mark.parametrize("n,share", [(2, 0), (3, 0), (5, 0), (63, 0), (64, 0), (65, 0), (129, 0),
                                      (296, 0), (297, 0), (512, 0), (513, 0), (1024, 0), (1025, 0),
-                                     (1537, 0), (2048, 0), (2049, 0), (64, 1), (301, 3),
+                                     (1537, 0), (2048, 0), (2049, 0), (300, 8), (64, 1), (301, 3),
                                      (613, 24), (901, 24)])
 def test_resident_tridiagonalisation(n, share):
     A = _matrix(n, n)
