@@ -12,7 +12,7 @@
 // Method (Hestenes 1958; the parallel ordering of Brent & Luk 1985):
 //   G = A, V = I.  A sweep visits every column pair (p, q) once, in n'-1
 //   rounds of n'/2 disjoint pairs (n' = n rounded up to even; the round-robin
-//   "circle" ordering), one warp per pair:
+//   "circle" ordering), eight lanes per pair:
 //     alpha = g_p.g_p, beta = g_q.g_q, gamma = g_p.g_q;
 //     if |gamma| > tol sqrt(alpha beta):
 //       zeta = (beta - alpha) / (2 gamma), t = sign(zeta) / (|zeta| + sqrt(1 + zeta^2)),
@@ -36,7 +36,6 @@
 namespace imcom {
 namespace {
 
-constexpr int JAC_THREADS = 512;
 constexpr int JAC_MAX = IMCOM_JACOBI_MAX_N;
 constexpr int JAC_MAX_SWEEPS = 60;
 
@@ -46,91 +45,144 @@ __device__ __forceinline__ double jwarp_sum(double v) {
   return v;
 }
 
+// Columns in shared memory start 64 bytes apart modulo 128, so that eight rows
+// of four consecutive columns take two wavefronts.
+__host__ __device__ inline int jac_ld(int n) { return (n + 7) / 16 * 16 + 8; }
+
 // Matrix b of the batch: A_b at A + b strideA (column-major, lda); output
 // eigenvectors (ascending) at Q + b strideQ (ldq), eigenvalues at
 // L + b strideL.  status[b] = sweeps used, or -1 if it did not converge.
-__global__ void __launch_bounds__(JAC_THREADS, 1)
+//
+// A round is a chain (columns from shared memory, three sums, square roots and
+// divisions, columns back), so each pair's work is spread over as few
+// instructions as its sums allow: a warp takes four pairs at once, eight lanes
+// each, and every lane rows i + 8 a + 32 c, with an accumulator per a.  Adding
+// these (0 with 2, 1 with 3) and then lanes is the tree of a whole warp on one
+// pair, so the results are the same to the bit.  Columns stay in registers
+// between the sums and the rotation, and the rotations' columns are on their way
+// while the angle is formed.  The test takes the square root only where the
+// squares do not decide it, and lanes that do not rotate divide 1 by 1 (a zero
+// or infinite operand sends the whole warp through the division's slow path).
+// A call with one system of 75 (20 sweeps of 75 rounds): 5.2 ms with a warp per
+// pair, three pairs one after another, 2.0 now; of 112, 64 systems: 19.3 -> 8.4.
+template <int C>  // chunks of 32 rows
+__global__ void __launch_bounds__(32 * (((C < 4 ? 32 * C : JAC_MAX) + 7) / 8), 1)
 jacobi_kernel(const double* __restrict__ A, long long lda, long long strideA, int n,
               double* __restrict__ Q, long long ldq, long long strideQ,
               double* __restrict__ L, long long strideL, int* __restrict__ status) {
   extern __shared__ __align__(16) double jsm[];
-  double* G = jsm;                   // n x n, column-major, ld n
-  double* V = G + (size_t)n * n;     // n x n
-  double* lam = V + (size_t)n * n;   // n
-  __shared__ int rotated;
+  const int ld = jac_ld(n);
+  double* G = jsm;                   // n columns, column-major
+  double* V = G + (size_t)n * ld;
+  double* lam = V + (size_t)n * ld;  // n
   const int b = blockIdx.x, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  constexpr int NW = JAC_THREADS / 32;
+  const int NT = blockDim.x, NW = NT / 32;
   const double* Ab = A + (size_t)b * strideA;
-  for (int idx = tid; idx < n * n; idx += JAC_THREADS) {
+  for (int idx = tid; idx < n * n; idx += NT) {
     const int r = idx % n, c = idx / n;
-    G[idx] = Ab[r + (long long)c * lda];
-    V[idx] = (r == c) ? 1.0 : 0.0;
+    G[r + c * ld] = Ab[r + (long long)c * lda];
+    V[r + c * ld] = (r == c) ? 1.0 : 0.0;
   }
   const int np = n + (n & 1);  // players of the round-robin (one idle when n is odd)
   const int m = np - 1;        // rotating players; player m is fixed
   const double tol = 2.0 * 1.1102230246251565e-16 * sqrt((double)n);
+  const int k = wid * 4 + (lane >> 3), r0 = lane & 7;
   int sweeps = 0;
   bool converged = (n <= 1);
   __syncthreads();
   while (!converged && sweeps < JAC_MAX_SWEEPS) {
-    if (tid == 0) rotated = 0;
-    __syncthreads();
+    bool rotated = false;
+    // round s: (m, s) and ((s + k) mod m, (s - k) mod m), k = 1 .. np/2 - 1
+    int up = k % m, dn = (m - up) % m;
     for (int s = 0; s < m; ++s) {
-      // round s: (m, s) and ((s + k) mod m, (s - k) mod m), k = 1 .. np/2 - 1
-      for (int k = wid; k < np / 2; k += NW) {
-        int p, q;
-        if (k == 0) {
-          p = s;
-          q = m;
-        } else {
-          p = (s + k) % m;
-          q = (s - k + m) % m;
+      const int p = k == 0 ? s : min(up, dn), q = k == 0 ? m : max(up, dn);
+      if (++up == m) up = 0;
+      if (++dn == m) dn = 0;
+      const bool on = k < np / 2 && q < n;  // not the idle player's
+      double* gp = G + p * ld + r0;
+      double* gq = G + q * ld + r0;
+      double x[4 * C], y[4 * C];
+#pragma unroll
+      for (int e = 0; e < 4 * C; ++e) {
+        const bool in = on && (e < 4 * C - 4 || r0 + 8 * e < n);
+        x[e] = in ? gp[8 * e] : 0.0;
+        y[e] = in ? gq[8 * e] : 0.0;
+      }
+      double al[4], be[4], ga[4];
+#pragma unroll
+      for (int a = 0; a < 4; ++a) {
+        al[a] = be[a] = ga[a] = 0.0;
+#pragma unroll
+        for (int c = 0; c < C; ++c) {
+          al[a] = fma(x[4 * c + a], x[4 * c + a], al[a]);
+          be[a] = fma(y[4 * c + a], y[4 * c + a], be[a]);
+          ga[a] = fma(x[4 * c + a], y[4 * c + a], ga[a]);
         }
-        if (p > q) {
-          const int t0 = p;
-          p = q;
-          q = t0;
-        }
-        if (q >= n) continue;  // the idle player
-        double* gp = G + (size_t)p * n;
-        double* gq = G + (size_t)q * n;
-        double al = 0.0, be = 0.0, ga = 0.0;
-        for (int r = lane; r < n; r += 32) {
-          const double x = gp[r], y = gq[r];
-          al = fma(x, x, al);
-          be = fma(y, y, be);
-          ga = fma(x, y, ga);
-        }
-        al = jwarp_sum(al);
-        be = jwarp_sum(be);
-        ga = jwarp_sum(ga);
-        if (ga == 0.0 || !(fabs(ga) > tol * sqrt(al * be))) continue;
-        const double zeta = (be - al) / (2.0 * ga);
+      }
+      double sa = (al[0] + al[2]) + (al[1] + al[3]);
+      double sb = (be[0] + be[2]) + (be[1] + be[3]);
+      double sg = (ga[0] + ga[2]) + (ga[1] + ga[3]);
+#pragma unroll
+      for (int o = 4; o > 0; o >>= 1) {
+        sa += __shfl_xor_sync(0xffffffffu, sa, o);
+        sb += __shfl_xor_sync(0xffffffffu, sb, o);
+        sg += __shfl_xor_sync(0xffffffffu, sg, o);
+      }
+      // |sg| > tol sqrt(sa sb): by the squares unless they are within 1e-6 or
+      // near the ends of the range
+      const double pr = sa * sb, lim = (tol * tol) * pr, g2 = sg * sg;
+      bool rot = g2 > lim;
+      if (on && (!(fabs(g2 - lim) > 1e-6 * lim) || !(pr > 1e-240 && pr < 1e290) || !(g2 < 1e290)))
+        rot = sg != 0.0 && fabs(sg) > tol * sqrt(pr);
+      rot = rot && on;
+      if (__any_sync(0xffffffffu, rot)) {
+        double* vp = V + p * ld + r0;
+        double* vq = V + q * ld + r0;
+        constexpr int H = C < 4 ? 4 * C : 8;  // rows of V held at a time
+        double u[H], w[H];
+        auto load = [&](int e0) {
+#pragma unroll
+          for (int e = 0; e < H; ++e) {
+            const bool in = rot && (e0 + e < 4 * C - 4 || r0 + 8 * (e0 + e) < n);
+            u[e] = in ? vp[8 * (e0 + e)] : 0.0;
+            w[e] = in ? vq[8 * (e0 + e)] : 0.0;
+          }
+        };
+        load(0);
+        // lanes that do not rotate divide 1 by 1
+        const double zeta = (rot ? sb - sa : 1.0) / (rot ? 2.0 * sg : 1.0);
         const double t = copysign(1.0, zeta) / (fabs(zeta) + sqrt(1.0 + zeta * zeta));
         const double c = 1.0 / sqrt(1.0 + t * t), sn = c * t;
-        double* vp = V + (size_t)p * n;
-        double* vq = V + (size_t)q * n;
-        for (int r = lane; r < n; r += 32) {
-          const double x = gp[r], y = gq[r];
-          gp[r] = c * x - sn * y;
-          gq[r] = sn * x + c * y;
-          const double u = vp[r], w = vq[r];
-          vp[r] = c * u - sn * w;
-          vq[r] = sn * u + c * w;
+#pragma unroll
+        for (int e = 0; e < 4 * C; ++e) {
+          if (rot && (e < 4 * C - 4 || r0 + 8 * e < n)) {
+            gp[8 * e] = c * x[e] - sn * y[e];
+            gq[8 * e] = sn * x[e] + c * y[e];
+          }
         }
-        if (lane == 0) rotated = 1;
+#pragma unroll
+        for (int e0 = 0; e0 < 4 * C; e0 += H) {
+          if (e0) load(e0);
+#pragma unroll
+          for (int e = 0; e < H; ++e) {
+            if (rot && (e0 + e < 4 * C - 4 || r0 + 8 * (e0 + e) < n)) {
+              vp[8 * (e0 + e)] = c * u[e] - sn * w[e];
+              vq[8 * (e0 + e)] = sn * u[e] + c * w[e];
+            }
+          }
+        }
+        rotated |= rot;
       }
       __syncthreads();
     }
     ++sweeps;
-    converged = (rotated == 0);
-    __syncthreads();  // every thread has read `rotated` before the next sweep resets it
+    converged = !__syncthreads_or(rotated);
   }
   if (tid == 0) status[b] = converged ? sweeps : -1;
   // lambda_i = v_i . g_i
   for (int i = wid; i < n; i += NW) {
     double acc = 0.0;
-    for (int r = lane; r < n; r += 32) acc = fma(V[(size_t)i * n + r], G[(size_t)i * n + r], acc);
+    for (int r = lane; r < n; r += 32) acc = fma(V[i * ld + r], G[i * ld + r], acc);
     acc = jwarp_sum(acc);
     if (lane == 0) lam[i] = acc;
   }
@@ -148,11 +200,12 @@ jacobi_kernel(const double* __restrict__ A, long long lda, long long strideA, in
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) rank += __shfl_xor_sync(0xffffffffu, rank, o);
     if (lane == 0) Lb[rank] = li;
-    for (int r = lane; r < n; r += 32) Qb[r + (long long)rank * ldq] = V[(size_t)i * n + r];
+    for (int r = lane; r < n; r += 32) Qb[r + (long long)rank * ldq] = V[i * ld + r];
   }
 }
 
-size_t jacobi_smem(int n) { return (2 * (size_t)n * n + n) * sizeof(double); }
+size_t jacobi_smem(int n) { return (2 * (size_t)n * jac_ld(n) + n) * sizeof(double); }
+
 
 int launch_jacobi(imcom_ctx* ctx, const double* A, long long lda, long long strideA, int n,
                   int count, double* Q, long long ldq, long long strideQ, double* L,
@@ -161,11 +214,19 @@ int launch_jacobi(imcom_ctx* ctx, const double* A, long long lda, long long stri
     return set_err(ctx, IMCOM_ERR_STATE,
                    "the Jacobi eigensolver takes n <= %d (shared memory); n = %d", JAC_MAX, n);
   const size_t smem = jacobi_smem(n);
-  // the largest size's need: the attribute is process-wide (see usum.cuh)
-  IMC_CUDA(cudaFuncSetAttribute(jacobi_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)jacobi_smem(JAC_MAX)));
-  jacobi_kernel<<<count, JAC_THREADS, smem, ctx->stream>>>(A, lda, strideA, n, Q, ldq, strideQ, L,
-                                                           strideL, status);
+  const int threads = 32 * ((n + 7) / 8);  // four pairs per warp
+  auto launch = [&](auto kernel) {
+    // the largest size's need: the attribute is process-wide (see usum.cuh)
+    IMC_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)jacobi_smem(JAC_MAX)));
+    kernel<<<count, threads, smem, ctx->stream>>>(A, lda, strideA, n, Q, ldq, strideQ, L, strideL,
+                                                  status);
+    return 0;
+  };
+  IMC_TRY(n <= 32   ? launch(jacobi_kernel<1>)
+          : n <= 64 ? launch(jacobi_kernel<2>)
+          : n <= 96 ? launch(jacobi_kernel<3>)
+                    : launch(jacobi_kernel<4>));
   IMC_LAUNCH();
   return 0;
 }
