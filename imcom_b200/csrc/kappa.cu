@@ -640,161 +640,317 @@ __global__ void __launch_bounds__(LB_WARPS * 32, 7) learned_fused_kernel(BisectA
 }
 
 // ---------------------------------------------------------------------------
-// Training: forward + backward for tiles of 32 samples per CTA, bf16
-// activations, fp32 accumulation; per-CTA gradient partials are added to a
-// global fp32 gradient with one atomic per parameter per CTA.
+// Training: forward + backward, bf16 weights and activations, fp32 sums,
+// gradients and Adam state.
 // Loss per sample: (o0 - t)^2 + 0.25 (o1 - log(|o0 - t| + 0.01))^2, the second
 // term with the target held fixed (it fits the log of the first head's error).
+//
+// One cooperative launch runs an epoch.  A CTA takes tiles of 32 samples of
+// each batch, sums its gradients in registers and adds them to the batch's
+// gradient with one atomic per parameter; past the grid barrier every CTA reads
+// the whole gradient and takes the same Adam step on its own copy of the
+// parameters: fp32 parameters and moments in registers, the rounded weights in
+// shared memory.  Three gradient buffers in turn leave one to clear.
+// What bounds it: shared-memory reads of the 64 x 64 layer (about 6000 cycles a
+// tile), the barrier and the chain of small layers.  A step of 512 samples: 29
+// us as three launches (clear, gradient, Adam) with layer 2 reading its weights
+// 64 floats apart, 13 now.  Tiles of eight samples are as fast at 512 samples, but
+// add up in other partial sums.
 // ---------------------------------------------------------------------------
-constexpr int TB = 32;  // samples per CTA tile
+constexpr int TB = 32;              // samples per tile
+constexpr int TRAIN_THREADS = 512;  // thread: unit u = tid % 64 of RPT rows tid / 64 + RG i
+constexpr int RG = TRAIN_THREADS / NH, RPT = TB / RG;
+constexpr int PPT = (NPARAM + TRAIN_THREADS - 1) / TRAIN_THREADS;  // parameters per thread
+constexpr int GSTRIDE = (NPARAM + 3) / 4 * 4;                      // a gradient buffer
 
-__global__ void __launch_bounds__(256) mlp_grad_kernel(const float* __restrict__ params,
-                                                       const float* __restrict__ feat, int nall,
-                                                       const float* __restrict__ target,
-                                                       const int* __restrict__ idx, int nb,
-                                                       float* __restrict__ grad,
-                                                       float* __restrict__ loss) {
-  __shared__ float sW1[NH * NF], sW2[NH * NH], sW3[NO * NH], sb1[NH], sb2[NH], sb3[NO];
-  __shared__ float X0[TB][NF + 1];
-  // H1 and H2 hold the activations, then (in place) their gradients
-  __shared__ float H1[TB][NH + 1], H2[TB][NH + 1];
+struct TrainArgs {
+  float* params;  // packed
+  const float* feat;
+  int nall;
+  const float* target;
+  const int* idx;     // order of the samples, or null
+  int nsamples, batch;
+  float* grad;        // GSTRIDE floats, zero; three of them when training
+  float* loss;
+  float *m1, *m2;     // Adam moments
+  const float2* c12;  // per step: 1 - b1^step, 1 - b2^step
+  float lr, b1, b2;
+  unsigned* arrived;  // barrier count, zero at the launch
+  int* err;
+  long long spin;
+};
+
+template <bool TRAIN>
+__global__ void __launch_bounds__(TRAIN_THREADS, 1) mlp_train_kernel(TrainArgs a) {
+  __shared__ float sW1[NF][NH];           // transposed
+  __shared__ float sW2[NH][NH + 1];       // transposed
+  __shared__ float sW3[NO][NH + 1], sb1[NH], sb2[NH], sb3[NO];
+  __shared__ float X0[TB][NF], sy[TB];
+  // activations, and the gradients before the ReLUs (layer 1's in place of H2)
+  __shared__ __align__(16) float H1[TB][NH], D2[TB][NH];
+  __shared__ float H2[TB][NH + 1];
   __shared__ float DO[TB][NO];
-  __shared__ float sloss[256];
+  __shared__ int s_stop;
   const int tid = threadIdx.x;
-  for (int q = tid; q < NH * NF; q += 256) sW1[q] = bf16r(params[OFF_W1 + q]);
-  for (int q = tid; q < NH * NH; q += 256) sW2[q] = bf16r(params[OFF_W2 + q]);
-  for (int q = tid; q < NO * NH; q += 256) sW3[q] = bf16r(params[OFF_W3 + q]);
-  for (int q = tid; q < NH; q += 256) {
-    sb1[q] = params[OFF_B1 + q];
-    sb2[q] = params[OFF_B2 + q];
-  }
-  if (tid < NO) sb3[tid] = params[OFF_B3 + tid];
-  const int s0 = blockIdx.x * TB;
-  for (int q = tid; q < TB * NF; q += 256) {
-    int r = q / NF, k = q % NF, s = s0 + r;
-    float v = 0.0f;
-    if (s < nb) {
-      int g = idx ? idx[s] : s;
-      v = bf16r(feat[(size_t)k * nall + g]);
-    }
-    X0[r][k] = v;
-  }
-  __syncthreads();
-  // layer 1
-  for (int q = tid; q < TB * NH; q += 256) {
-    int r = q / NH, u = q % NH;
-    float s = sb1[u];
+  const int u = tid % NH, rg = tid / NH;
+  const int G = gridDim.x, steps = (a.nsamples + a.batch - 1) / a.batch;
+  float p[PPT], m1[PPT], m2[PPT];
+  auto store_weight = [&](int q, float v) {
+    if (q < OFF_B1) sW1[q % NF][q / NF] = bf16r(v);
+    else if (q < OFF_W2) sb1[q - OFF_B1] = v;
+    else if (q < OFF_B2) sW2[(q - OFF_W2) % NH][(q - OFF_W2) / NH] = bf16r(v);
+    else if (q < OFF_W3) sb2[q - OFF_B2] = v;
+    else if (q < OFF_B3) sW3[(q - OFF_W3) / NH][(q - OFF_W3) % NH] = bf16r(v);
+    else sb3[q - OFF_B3] = v;
+  };
 #pragma unroll
-    for (int k = 0; k < NF; ++k) s = fmaf(sW1[u * NF + k], X0[r][k], s);
-    H1[r][u] = bf16r(fmaxf(s, 0.0f));
+  for (int i = 0; i < PPT; ++i) {
+    const int q = tid + TRAIN_THREADS * i;
+    p[i] = m1[i] = m2[i] = 0.0f;
+    if (q < NPARAM) {
+      p[i] = a.params[q];
+      if (TRAIN) {
+        m1[i] = a.m1[q];
+        m2[i] = a.m2[q];
+      }
+    }
   }
-  __syncthreads();
-  // layer 2
-  for (int q = tid; q < TB * NH; q += 256) {
-    int r = q / NH, u = q % NH;
-    float s = sb2[u];
-    for (int v = 0; v < NH; ++v) s = fmaf(sW2[u * NH + v], H1[r][v], s);
-    H2[r][u] = bf16r(fmaxf(s, 0.0f));
-  }
-  __syncthreads();
-  // output, loss and d loss / d output
-  float lsum = 0.0f;
-  if (tid < TB) {
-    int r = tid, s = s0 + r;
-    float o[NO];
 #pragma unroll
-    for (int j = 0; j < NO; ++j) {
-      float acc = sb3[j];
-      for (int v = 0; v < NH; ++v) acc = fmaf(sW3[j * NH + v], H2[r][v], acc);
-      o[j] = acc;
-    }
-    float d0 = 0.0f, d1 = 0.0f;
-    if (s < nb) {
-      int g = idx ? idx[s] : s;
-      float e = o[0] - target[g];
-      float lt = logf(fabsf(e) + 0.01f);
-      float e1 = o[1] - lt;
-      lsum = e * e + 0.25f * e1 * e1;
-      d0 = 2.0f * e;
-      d1 = 0.5f * e1;
-    }
-    DO[r][0] = d0;
-    DO[r][1] = d1;
-  }
-  sloss[tid] = lsum;
-  __syncthreads();
-  // dW3, db3 (need H2 before it is overwritten)
-  for (int q = tid; q < NO * NH; q += 256) {
-    int j = q / NH, v = q % NH;
-    float g = 0.0f;
-    for (int r = 0; r < TB; ++r) g = fmaf(DO[r][j], H2[r][v], g);
-    atomicAdd(&grad[OFF_W3 + q], g);
-  }
-  if (tid < NO) {
-    float g = 0.0f;
-    for (int r = 0; r < TB; ++r) g += DO[r][tid];
-    atomicAdd(&grad[OFF_B3 + tid], g);
-  }
-  __syncthreads();
-  // H2 <- d(pre-activation 2) = (W3^T dO) masked by ReLU, in place
-  for (int q = tid; q < TB * NH; q += 256) {
-    int r = q / NH, u = q % NH;
-    float g = DO[r][0] * sW3[u] + DO[r][1] * sW3[NH + u];
-    H2[r][u] = H2[r][u] > 0.0f ? g : 0.0f;
-  }
-  __syncthreads();
-  // dW2 = dH2^T H1, db2 (need H1 before it is overwritten)
-  for (int q = tid; q < NH * NH; q += 256) {
-    int u = q / NH, v = q % NH;
-    float g = 0.0f;
-    for (int r = 0; r < TB; ++r) g = fmaf(H2[r][u], H1[r][v], g);
-    atomicAdd(&grad[OFF_W2 + q], g);
-  }
-  for (int q = tid; q < NH; q += 256) {
-    float g = 0.0f;
-    for (int r = 0; r < TB; ++r) g += H2[r][q];
-    atomicAdd(&grad[OFF_B2 + q], g);
-  }
-  __syncthreads();
-  // H1 <- d(pre-activation 1) = (W2^T dH2) masked by ReLU, in place
-  for (int q = tid; q < TB * NH; q += 256) {
-    int r = q / NH, v = q % NH;
-    float g = 0.0f;
-    for (int u = 0; u < NH; ++u) g = fmaf(sW2[u * NH + v], H2[r][u], g);
-    H1[r][v] = H1[r][v] > 0.0f ? g : 0.0f;
-  }
-  __syncthreads();
-  // dW1 = dH1^T X0, db1
-  for (int q = tid; q < NH * NF; q += 256) {
-    int u = q / NF, k = q % NF;
-    float g = 0.0f;
-    for (int r = 0; r < TB; ++r) g = fmaf(H1[r][u], X0[r][k], g);
-    atomicAdd(&grad[OFF_W1 + q], g);
-  }
-  for (int q = tid; q < NH; q += 256) {
-    float g = 0.0f;
-    for (int r = 0; r < TB; ++r) g += H1[r][q];
-    atomicAdd(&grad[OFF_B1 + q], g);
-  }
-  for (int w = 128; w > 0; w >>= 1) {
-    __syncthreads();
-    if (tid < w) sloss[tid] += sloss[tid + w];
-  }
-  if (tid == 0) atomicAdd(loss, sloss[0]);
-}
+  for (int i = 0; i < PPT; ++i)
+    if (tid + TRAIN_THREADS * i < NPARAM) store_weight(tid + TRAIN_THREADS * i, p[i]);
+  if (tid == 0) s_stop = 0;
 
-// Adam step on fp32 master parameters with the batch-mean gradient.
-__global__ void adam_kernel(float* __restrict__ params, const float* __restrict__ grad,
-                            float* __restrict__ m1, float* __restrict__ m2, float lr, float b1,
-                            float b2, float c1, float c2, float inv_batch) {
-  int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= NPARAM) return;
-  float g = grad[q] * inv_batch;
-  float a = b1 * m1[q] + (1.0f - b1) * g;
-  float b = b2 * m2[q] + (1.0f - b2) * g * g;
-  m1[q] = a;
-  m2[q] = b;
-  params[q] -= lr * (a / c1) / (sqrtf(b / c2) + 1e-8f);
+  static_assert(RG == NF / 2 + 2, "row groups: six of dW1, db1, db2");
+  static_assert(64 + TB * NF + TB <= TRAIN_THREADS, "a thread per feature and target");
+  // This CTA's tiles in order.  A sample's index is on its way two tiles ahead
+  // and its data one ahead: threads 64 .. 447 hold a feature of a sample each,
+  // 448 .. 479 a target.
+  struct Item {
+    int step, tile;
+  };
+  auto settle = [&](Item& it) {
+    while (it.step < steps && it.tile * TB >= min(a.batch, a.nsamples - it.step * a.batch)) {
+      ++it.step;
+      it.tile = blockIdx.x;
+    }
+  };
+  constexpr int FEATS = TB * NF;
+  const int lt = tid - 64;
+  const int lrow = lt < FEATS ? max(lt, 0) / NF : (lt - FEATS) % TB, lk = max(lt, 0) % NF;
+  Item at{0, (int)blockIdx.x};
+  settle(at);
+  int g_next = -1;
+  float x_next = 0.0f;
+  auto fetch_index = [&]() {
+    g_next = -1;
+    if (lt >= 0 && lt < FEATS + TB && at.step < steps) {
+      const int s = at.tile * TB + lrow, first = at.step * a.batch;
+      if (s < min(a.batch, a.nsamples - first)) g_next = a.idx ? a.idx[first + s] : first + s;
+    }
+    at.tile += G;
+    settle(at);
+  };
+  auto fetch_data = [&]() {
+    x_next = 0.0f;
+    if (g_next >= 0)
+      x_next = lt < FEATS ? bf16r(a.feat[(size_t)lk * a.nall + g_next]) : a.target[g_next];
+    fetch_index();
+  };
+  fetch_index();
+  fetch_data();
+
+  const int tu = tid / 32, tv = tid % 32;  // dW2: units 4 tu .., inputs tv and tv + 32
+  float lsum = 0.0f;
+  for (int step = 0; step < steps; ++step) {
+    const int nb = min(a.batch, a.nsamples - step * a.batch);
+    float gW2[4][2] = {}, gW1[2] = {}, gb = 0.0f, gW3 = 0.0f;
+    for (int tile = blockIdx.x; tile * TB < nb; tile += G) {
+      if (lt >= 0 && lt < FEATS) X0[lrow][lk] = x_next;
+      else if (lt >= FEATS && lt < FEATS + TB) sy[lrow] = x_next;
+      __syncthreads();
+      if (tile + G < (nb + TB - 1) / TB) fetch_data();
+      // layer 1
+      float h1[RPT];
+#pragma unroll
+      for (int i = 0; i < RPT; ++i) {
+        float s = sb1[u];
+#pragma unroll
+        for (int k = 0; k < NF; ++k) s = fmaf(sW1[k][u], X0[rg + RG * i][k], s);
+        h1[i] = bf16r(fmaxf(s, 0.0f));
+        H1[rg + RG * i][u] = h1[i];
+      }
+      __syncthreads();
+      // layer 2
+      float h2[RPT];
+#pragma unroll
+      for (int i = 0; i < RPT; ++i) h2[i] = sb2[u];
+#pragma unroll 4
+      for (int v = 0; v < NH; v += 4) {
+        const float w0 = sW2[v][u], w1 = sW2[v + 1][u], w2 = sW2[v + 2][u], w3 = sW2[v + 3][u];
+#pragma unroll
+        for (int i = 0; i < RPT; ++i) {
+          const float4 h = *(const float4*)&H1[rg + RG * i][v];
+          h2[i] = fmaf(w3, h.w, fmaf(w2, h.z, fmaf(w1, h.y, fmaf(w0, h.x, h2[i]))));
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < RPT; ++i) {
+        h2[i] = bf16r(fmaxf(h2[i], 0.0f));
+        H2[rg + RG * i][u] = h2[i];
+      }
+      __syncthreads();
+      // output, loss and d loss / d output: a lane per sample and output
+      if (tid < NO * TB) {
+        const int r = tid / NO, j = tid % NO;
+        float o = sb3[j];
+#pragma unroll 16
+        for (int v = 0; v < NH; ++v) o = fmaf(sW3[j][v], H2[r][v], o);
+        const float o1 = __shfl_down_sync(0xffffffffu, o, 1);
+        if (j == 0) {
+          float d0 = 0.0f, d1 = 0.0f;
+          if (tile * TB + r < nb) {
+            const float e = o - sy[r];
+            const float ltar = logf(fabsf(e) + 0.01f);
+            const float e1 = o1 - ltar;
+            lsum += e * e + 0.25f * e1 * e1;
+            d0 = 2.0f * e;
+            d1 = 0.5f * e1;
+          }
+          DO[r][0] = d0;
+          DO[r][1] = d1;
+        }
+      }
+      __syncthreads();
+#pragma unroll
+      for (int i = 0; i < RPT; ++i) {
+        const int r = rg + RG * i;
+        const float g = DO[r][0] * sW3[0][u] + DO[r][1] * sW3[1][u];
+        D2[r][u] = h2[i] > 0.0f ? g : 0.0f;
+      }
+      if (tid < NO * NH) {
+#pragma unroll 8
+        for (int r = 0; r < TB; ++r) gW3 = fmaf(DO[r][rg], H2[r][u], gW3);
+      } else if (tid < NO * NH + NO) {
+#pragma unroll 8
+        for (int r = 0; r < TB; ++r) gW3 += DO[r][tid - NO * NH];
+      }
+      __syncthreads();
+      // dW2 = dH2^T H1, and db2
+#pragma unroll 4
+      for (int r = 0; r < TB; ++r) {
+        const float4 d = *(const float4*)&D2[r][4 * tu];
+        const float dd[4] = {d.x, d.y, d.z, d.w}, hh[2] = {H1[r][tv], H1[r][tv + 32]};
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int j = 0; j < 2; ++j) gW2[i][j] = fmaf(dd[i], hh[j], gW2[i][j]);
+      }
+      if (rg == RG - 1) {
+#pragma unroll 8
+        for (int r = 0; r < TB; ++r) gb += D2[r][u];
+      }
+      // dH1 = W2^T dH2 where the ReLU passes
+      float d1[RPT] = {};
+#pragma unroll 4
+      for (int v = 0; v < NH; v += 4) {
+        const float w0 = sW2[u][v], w1 = sW2[u][v + 1], w2 = sW2[u][v + 2], w3 = sW2[u][v + 3];
+#pragma unroll
+        for (int i = 0; i < RPT; ++i) {
+          const float4 d = *(const float4*)&D2[rg + RG * i][v];
+          d1[i] = fmaf(w3, d.w, fmaf(w2, d.z, fmaf(w1, d.y, fmaf(w0, d.x, d1[i]))));
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < RPT; ++i) H2[rg + RG * i][u] = h1[i] > 0.0f ? d1[i] : 0.0f;
+      __syncthreads();
+      // dW1 = dH1^T X0, and db1
+      if (rg < NF / 2) {
+#pragma unroll 8
+        for (int r = 0; r < TB; ++r) {
+          const float d = H2[r][u];
+          gW1[0] = fmaf(d, X0[r][2 * rg], gW1[0]);
+          gW1[1] = fmaf(d, X0[r][2 * rg + 1], gW1[1]);
+        }
+      } else if (rg == NF / 2) {
+#pragma unroll 8
+        for (int r = 0; r < TB; ++r) gb += H2[r][u];
+      }
+      __syncthreads();
+    }
+    float* grad = a.grad + (TRAIN ? step % 3 : 0) * GSTRIDE;
+    if (blockIdx.x * TB < nb) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+          atomicAdd(grad + OFF_W2 + (4 * tu + i) * NH + tv + 32 * j, gW2[i][j]);
+      if (rg < NF / 2) {
+        atomicAdd(grad + OFF_W1 + u * NF + 2 * rg, gW1[0]);
+        atomicAdd(grad + OFF_W1 + u * NF + 2 * rg + 1, gW1[1]);
+      } else if (rg == NF / 2) {
+        atomicAdd(grad + OFF_B1 + u, gb);
+      } else {
+        atomicAdd(grad + OFF_B2 + u, gb);
+      }
+      if (tid < NO * NH + NO) atomicAdd(grad + OFF_W3 + tid, gW3);
+    }
+    if (!TRAIN) break;
+    // grid barrier; the next tile's data is on its way meanwhile
+    __syncthreads();
+    if (tid == 0) {
+      __threadfence();
+      atomicAdd(a.arrived, 1u);
+    }
+    fetch_data();
+    if (tid == 0) {
+      const unsigned want = (unsigned)G * (step + 1);
+      long long it = 0;
+      unsigned have;
+      do {
+        asm volatile("ld.acquire.gpu.u32 %0, [%1];" : "=r"(have) : "l"(a.arrived) : "memory");
+      } while (have < want && ++it < a.spin);
+      if (have < want) {
+        atomicExch(a.err, 1);
+        s_stop = 1;
+      }
+      __threadfence();
+    }
+    __syncthreads();
+    if (s_stop) return;
+    const float2 c = a.c12[step];
+    const float inv = 1.0f / nb;
+    float gr[PPT];
+#pragma unroll
+    for (int i = 0; i < PPT; ++i) {
+      const int q = tid + TRAIN_THREADS * i;
+      gr[i] = q < NPARAM ? __ldcg(grad + q) : 0.0f;
+    }
+    // the buffer of the step before last (read by every CTA before this barrier)
+    float* old = a.grad + (step + 2) % 3 * GSTRIDE;
+    for (int q = blockIdx.x * TRAIN_THREADS + tid; q < NPARAM; q += G * TRAIN_THREADS) old[q] = 0.0f;
+#pragma unroll
+    for (int i = 0; i < PPT; ++i) {
+      const int q = tid + TRAIN_THREADS * i;
+      const float g = gr[i] * inv;
+      m1[i] = fmaf(a.b1, m1[i], (1.0f - a.b1) * g);
+      m2[i] = fmaf(a.b2, m2[i], (1.0f - a.b2) * g * g);
+      p[i] -= a.lr * (m1[i] / c.x) / (sqrtf(m2[i] / c.y) + 1e-8f);
+      if (q < NPARAM) store_weight(q, p[i]);
+    }
+    __syncthreads();
+  }
+  if (lsum != 0.0f) atomicAdd(a.loss, lsum);
+  if (TRAIN && blockIdx.x == 0) {
+#pragma unroll
+    for (int i = 0; i < PPT; ++i) {
+      const int q = tid + TRAIN_THREADS * i;
+      if (q < NPARAM) {
+        a.params[q] = p[i];
+        a.m1[q] = m1[i];
+        a.m2[q] = m2[i];
+      }
+    }
+  }
 }
 
 }  // namespace
@@ -956,6 +1112,11 @@ extern "C" int imcom_gpu_bisect_kappa_learned(imcom_ctx* ctx, int UnotS, double 
   return copy_pixel_outputs(ctx, K_out, US_out, nevals_out);
 }
 
+// CTAs of the training kernel: a tile of each batch at least, one per SM.
+static int train_grid(imcom_ctx* ctx, int batch) {
+  return std::max(1, std::min((batch + TB - 1) / TB, sm_count(ctx)));
+}
+
 // Gradient of the summed loss over `nsamples` samples at the given parameters
 // (the training kernel on one batch; used by the tests' gradient check).
 extern "C" int imcom_gpu_mlp_gradient(imcom_ctx* ctx, int nsamples, const float* feat,
@@ -968,24 +1129,29 @@ extern "C" int imcom_gpu_mlp_gradient(imcom_ctx* ctx, int nsamples, const float*
   if (!params) return -5;
   if (!grad_out) return -6;
   cudaSetDevice(ctx->device);
-  float *d = nullptr;
-  size_t need = ((size_t)NF * nsamples + nsamples + 2 * NPARAM + 64) * sizeof(float);
+  size_t need = ((size_t)NF * nsamples + nsamples + 2 * GSTRIDE + 64) * sizeof(float);
   IMC_TRY(ensure_buf(ctx, (void**)&ctx->train_buf, ctx->train_bytes, need));
-  d = (float*)ctx->train_buf;
-  float* dfeat = d;
+  float* dgrad = (float*)ctx->train_buf;  // 16-byte aligned, as the loss after it
+  float* dloss = dgrad + GSTRIDE;
+  float* dparams = dloss + 4;
+  float* dfeat = dparams + GSTRIDE;
   float* dtarget = dfeat + (size_t)NF * nsamples;
-  float* dparams = dtarget + nsamples;
-  float* dgrad = dparams + NPARAM;
-  float* dloss = dgrad + NPARAM;
   IMC_CUDA(cudaMemcpyAsync(dfeat, feat, (size_t)NF * nsamples * sizeof(float),
                            cudaMemcpyHostToDevice, ctx->stream));
   IMC_CUDA(cudaMemcpyAsync(dtarget, target, nsamples * sizeof(float), cudaMemcpyHostToDevice,
                            ctx->stream));
   IMC_CUDA(cudaMemcpyAsync(dparams, params, NPARAM * sizeof(float), cudaMemcpyHostToDevice,
                            ctx->stream));
-  IMC_CUDA(cudaMemsetAsync(dgrad, 0, (NPARAM + 1) * sizeof(float), ctx->stream));
-  mlp_grad_kernel<<<(nsamples + TB - 1) / TB, 256, 0, ctx->stream>>>(
-      dparams, dfeat, nsamples, dtarget, nullptr, nsamples, dgrad, dloss);
+  IMC_CUDA(cudaMemsetAsync(dgrad, 0, (GSTRIDE + 4) * sizeof(float), ctx->stream));
+  TrainArgs ta{};
+  ta.params = dparams;
+  ta.feat = dfeat;
+  ta.nall = ta.nsamples = ta.batch = nsamples;
+  ta.target = dtarget;
+  ta.grad = dgrad;
+  ta.loss = dloss;
+  mlp_train_kernel<false>
+      <<<train_grid(ctx, nsamples), TRAIN_THREADS, 0, ctx->stream>>>(ta);
   IMC_LAUNCH();
   IMC_CUDA(cudaMemcpyAsync(grad_out, dgrad, NPARAM * sizeof(float), cudaMemcpyDeviceToHost,
                            ctx->stream));
@@ -1009,25 +1175,35 @@ extern "C" int imcom_gpu_mlp_train(imcom_ctx* ctx, int nsamples, const float* fe
   if (!(lr > 0.0f)) return -7;
   if (!params) return -9;
   cudaSetDevice(ctx->device);
-  size_t need = ((size_t)NF * nsamples + nsamples + 4 * NPARAM + 64) * sizeof(float) +
-                (size_t)nsamples * sizeof(int);
+  batch = std::min(batch, nsamples);
+  const int steps = (nsamples + batch - 1) / batch;
+  // gradients (three, in turn) | moments | parameters | per epoch the loss, the
+  // barrier's count and its error | per-step bias corrections and the epoch's order |
+  // features | targets
+  size_t need = (6 * (size_t)GSTRIDE + 4 * (size_t)epochs + 2 * (size_t)steps +
+                 (size_t)(NF + 2) * nsamples) * sizeof(float);
   IMC_TRY(ensure_buf(ctx, (void**)&ctx->train_buf, ctx->train_bytes, need));
-  float* dfeat = (float*)ctx->train_buf;
+  float* dgrad = (float*)ctx->train_buf;
+  float* dm1 = dgrad + 3 * GSTRIDE;
+  float* dm2 = dm1 + GSTRIDE;
+  float* dparams = dm2 + GSTRIDE;
+  float* dctl = dparams + GSTRIDE;
+  float2* dc12 = (float2*)(dctl + 4 * (size_t)epochs);
+  int* didx = (int*)(dc12 + steps);
+  float* dfeat = (float*)(didx + nsamples);
   float* dtarget = dfeat + (size_t)NF * nsamples;
-  float* dparams = dtarget + nsamples;
-  float* dgrad = dparams + NPARAM;
-  float* dm1 = dgrad + NPARAM + 1;
-  float* dm2 = dm1 + NPARAM;
-  int* didx = (int*)(dm2 + NPARAM + 16);
   IMC_CUDA(cudaMemcpyAsync(dfeat, feat, (size_t)NF * nsamples * sizeof(float),
                            cudaMemcpyHostToDevice, ctx->stream));
   IMC_CUDA(cudaMemcpyAsync(dtarget, target, nsamples * sizeof(float), cudaMemcpyHostToDevice,
                            ctx->stream));
   IMC_CUDA(cudaMemcpyAsync(dparams, params, NPARAM * sizeof(float), cudaMemcpyHostToDevice,
                            ctx->stream));
-  IMC_CUDA(cudaMemsetAsync(dm1, 0, 2 * (NPARAM + 8) * sizeof(float), ctx->stream));
+  IMC_CUDA(cudaMemsetAsync(dm1, 0, 2 * GSTRIDE * sizeof(float), ctx->stream));
+  IMC_CUDA(cudaMemsetAsync(dctl, 0, 4 * (size_t)epochs * sizeof(float), ctx->stream));
   // shuffled order per epoch (host xorshift, reproducible from the seed)
-  std::vector<int> order(nsamples);
+  std::vector<int> host(2 * (size_t)steps + nsamples);
+  float* c12 = (float*)host.data();
+  int* order = host.data() + 2 * (size_t)steps;
   unsigned s = seed ? seed : 1u;
   auto rnd = [&]() {
     s ^= s << 13;
@@ -1037,33 +1213,37 @@ extern "C" int imcom_gpu_mlp_train(imcom_ctx* ctx, int nsamples, const float* fe
   };
   const float b1 = 0.9f, b2 = 0.999f;
   int step = 0;
-  std::vector<float> eloss(epochs, 0.0f);
-  float* dloss = dgrad + NPARAM;
+  TrainArgs ta{dparams, dfeat, nsamples, dtarget, didx, nsamples, batch, dgrad, nullptr, dm1, dm2,
+               dc12, lr, b1, b2, nullptr, nullptr, 20000000LL};
   for (int ep = 0; ep < epochs; ++ep) {
     for (int q = 0; q < nsamples; ++q) order[q] = q;
     for (int q = nsamples - 1; q > 0; --q) std::swap(order[q], order[rnd() % (q + 1)]);
-    IMC_CUDA(cudaMemcpyAsync(didx, order.data(), nsamples * sizeof(int), cudaMemcpyHostToDevice,
-                             ctx->stream));
-    IMC_CUDA(cudaMemsetAsync(dloss, 0, sizeof(float), ctx->stream));
-    for (int b0 = 0; b0 < nsamples; b0 += batch) {
-      const int nb = std::min(batch, nsamples - b0);
-      IMC_CUDA(cudaMemsetAsync(dgrad, 0, NPARAM * sizeof(float), ctx->stream));
-      mlp_grad_kernel<<<(nb + TB - 1) / TB, 256, 0, ctx->stream>>>(
-          dparams, dfeat, nsamples, dtarget, didx + b0, nb, dgrad, dloss);
-      IMC_LAUNCH();
+    for (int q = 0; q < steps; ++q) {
       ++step;
-      const float c1 = 1.0f - powf(b1, (float)step), c2 = 1.0f - powf(b2, (float)step);
-      adam_kernel<<<(NPARAM + 255) / 256, 256, 0, ctx->stream>>>(dparams, dgrad, dm1, dm2, lr, b1,
-                                                                b2, c1, c2, 1.0f / nb);
-      IMC_LAUNCH();
+      c12[2 * q] = 1.0f - powf(b1, (float)step);
+      c12[2 * q + 1] = 1.0f - powf(b2, (float)step);
     }
-    IMC_CUDA(cudaMemcpyAsync(&eloss[ep], dloss, sizeof(float), cudaMemcpyDeviceToHost,
+    IMC_CUDA(cudaMemcpyAsync(dc12, host.data(), host.size() * sizeof(int), cudaMemcpyHostToDevice,
                              ctx->stream));
+    IMC_CUDA(cudaMemsetAsync(dgrad, 0, 3 * GSTRIDE * sizeof(float), ctx->stream));
+    ta.loss = dctl + 4 * (size_t)ep;
+    ta.arrived = (unsigned*)(ta.loss + 1);
+    ta.err = (int*)(ta.loss + 2);
+    void* args[] = {&ta};
+    IMC_CUDA(cudaLaunchCooperativeKernel((void*)mlp_train_kernel<true>, train_grid(ctx, batch),
+                                         TRAIN_THREADS, args, 0, ctx->stream));
+    IMC_LAUNCH();
   }
+  std::vector<float> ctl(4 * (size_t)epochs);
+  IMC_CUDA(cudaMemcpyAsync(ctl.data(), dctl, ctl.size() * sizeof(float), cudaMemcpyDeviceToHost,
+                           ctx->stream));
   IMC_CUDA(cudaMemcpyAsync(params, dparams, NPARAM * sizeof(float), cudaMemcpyDeviceToHost,
                            ctx->stream));
   IMC_CUDA(cudaStreamSynchronize(ctx->stream));
+  for (int ep = 0; ep < epochs; ++ep)
+    if (ctl[4 * (size_t)ep + 2] != 0.0f)
+      return set_err(ctx, IMCOM_ERR_CUDA, "training's grid barrier timed out");
   if (loss_out)
-    for (int ep = 0; ep < epochs; ++ep) loss_out[ep] = eloss[ep] / nsamples;
+    for (int ep = 0; ep < epochs; ++ep) loss_out[ep] = ctl[4 * (size_t)ep] / nsamples;
   return 0;
 }
