@@ -264,33 +264,56 @@ struct Node {
   int s, n1, nm;  // first row, left child size, node size
 };
 
-// Tearing: d(s-1) -= |e(s-1)|, d(s) -= |e(s-1)| at every split point.
+// Tearing: d(s-1) -= |e(s-1)|, d(s) -= |e(s-1)| at every split point (a thread
+// each: leaves hold LEAF / 2 rows or more, so no two splits share one).
 __global__ void tear_kernel(double* dt, const double* e, const int* splits, int nsplit) {
-  if (blockIdx.x == 0 && threadIdx.x == 0)
-    for (int q = 0; q < nsplit; ++q) {
-      int s = splits[q];
-      double b = fabs(e[s - 1]);
-      dt[s - 1] -= b;
-      dt[s] -= b;
-    }
+  const int q = blockIdx.x * blockDim.x + threadIdx.x;
+  if (q >= nsplit) return;
+  const int s = splits[q];
+  const double b = fabs(e[s - 1]);
+  dt[s - 1] -= b;
+  dt[s] -= b;
+}
+
+// The rotation (c, sn) that annihilates a_pq: t = tan of the smaller angle, from
+// t = 2 a / (d + sign(d) sqrt(d^2 + 4 a^2)), d = a_qq - a_pp, where the squares
+// stay in range, else from theta = d / (2 a).
+__device__ __forceinline__ void jacobi_angle(double d, double a, double& c, double& sn) {
+  const double a2 = 2.0 * a, big = fmax(fabs(d), fabs(a2));
+  double t;
+  if (big > 1e-140 && big < 1e150) {
+    t = copysign(a2, a2 * copysign(1.0, d)) / (fabs(d) + sqrt(fma(d, d, a2 * a2)));
+  } else {
+    const double theta = d / a2;
+    t = copysign(1.0, theta) / (fabs(theta) + sqrt(1.0 + theta * theta));
+  }
+  c = rsqrt(fma(t, t, 1.0));
+  sn = t * c;
 }
 
 // Cyclic Jacobi on one leaf (tridiagonal block), sorted ascending output.
+// A round is a chain of two barriers, a square root, a division and a
+// reciprocal root: one warp forms the angles of the round's disjoint pairs, then
+// thread (i, j) applies those of pairs i and j to the 2 x 2 block of rows i and
+// columns j, and to Z.  Leaves of 18 (order 72): 182 us with the sweep's test and
+// the sort on one thread and four barriers a round, 68 now; 64 leaves of 23,
+// 297 -> 113.
 __global__ void __launch_bounds__(256) leaf_jacobi_kernel(const Node* nodes, const double* dt,
                                                           const double* e, double* w, double* Z,
                                                           long long ldz, int max_sweeps,
                                                           int* err) {
   const Node nd = nodes[blockIdx.x];
   const int m = nd.nm, s0 = nd.s;
+  constexpr int NP = LEAF / 2;
   __shared__ double Am[LEAF][LEAF + 1];
   __shared__ double Zm[LEAF][LEAF + 1];
-  __shared__ double cs[LEAF / 2][2];
-  __shared__ int pr[LEAF / 2][2];
-  __shared__ int s_done;
-  __shared__ double s_val[LEAF];
+  __shared__ double cs[NP][2];
+  __shared__ int pr[NP][2];
+  __shared__ double s_off[8], s_tot[8];
   __shared__ int s_idx[LEAF];
-  const int tid = threadIdx.x;
-  for (int q = tid; q < LEAF * LEAF; q += blockDim.x) {
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  static_assert(NP * NP == 256, "a thread per 2 x 2 block");
+  for (int q = tid; q < LEAF * LEAF; q += 256) {
     int r = q % LEAF, c = q / LEAF;
     double v = 0.0;
     if (r < m && c < m) {
@@ -305,98 +328,91 @@ __global__ void __launch_bounds__(256) leaf_jacobi_kernel(const Node* nodes, con
   const int mp = (m + 1) & ~1;  // even number of players (a dummy when m is odd)
   for (int sweep = 0; sweep < max_sweeps; ++sweep) {
     // convergence: off-diagonal mass below eps^2 of the total
-    if (tid == 0) {
+    {
       double off = 0.0, tot = 0.0;
-      for (int r = 0; r < m; ++r)
-        for (int c = 0; c < m; ++c) {
-          double v = Am[r][c] * Am[r][c];
-          tot += v;
-          if (r != c) off += v;
-        }
-      s_done = (off <= 64.0 * EPS * EPS * tot) ? 1 : 0;
+      for (int q = tid; q < LEAF * LEAF; q += 256) {
+        const double v = Am[q / LEAF][q % LEAF] * Am[q / LEAF][q % LEAF];
+        tot += v;
+        if (q / LEAF != q % LEAF) off += v;
+      }
+      off = warp_sum(off);
+      tot = warp_sum(tot);
+      if (lane == 0) {
+        s_off[wid] = off;
+        s_tot[wid] = tot;
+      }
+      __syncthreads();
+      off = tot = 0.0;
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        off += s_off[k];
+        tot += s_tot[k];
+      }
+      if (off <= 64.0 * EPS * EPS * tot) break;
     }
-    __syncthreads();
-    if (s_done) break;
+    // player x > 0 of round rnd is 1 + (x - 1 + rnd) mod (mp - 1); pair x meets mp - 1 - x
+    int pa = tid < mp / 2 ? tid : 0, pb = mp - 1 - pa;
     for (int rnd = 0; rnd < mp - 1; ++rnd) {
       if (tid < mp / 2) {
-        auto idx = [&](int x) { return x == 0 ? 0 : 1 + (x - 1 + rnd) % (mp - 1); };
-        int p = idx(tid), q = idx(mp - 1 - tid);
-        if (p > q) { int tt = p; p = q; q = tt; }
+        const int p = min(pa, pb), q = max(pa, pb);
         double c = 1.0, sn = 0.0;
         if (q < m) {
-          double apq = Am[p][q];
-          if (apq != 0.0) {
-            double theta = (Am[q][q] - Am[p][p]) / (2.0 * apq);
-            double tt = copysign(1.0, theta) / (fabs(theta) + sqrt(1.0 + theta * theta));
-            c = 1.0 / sqrt(1.0 + tt * tt);
-            sn = tt * c;
-          }
+          const double apq = Am[p][q];
+          if (apq != 0.0) jacobi_angle(Am[q][q] - Am[p][p], apq, c, sn);
         }
         pr[tid][0] = p;
         pr[tid][1] = q;
         cs[tid][0] = c;
         cs[tid][1] = sn;
+        if (tid > 0 && ++pa == mp) pa = 1;
+        if (++pb == mp) pb = 1;
       }
       __syncthreads();
-      // columns: A <- A J, Z <- Z J
-      for (int item = tid; item < (mp / 2) * LEAF; item += blockDim.x) {
-        int pi = item / LEAF, r = item % LEAF;
-        int p = pr[pi][0], q = pr[pi][1];
-        if (q >= m || r >= m) continue;
-        double c = cs[pi][0], sn = cs[pi][1];
-        double ap = Am[r][p], aq = Am[r][q];
-        Am[r][p] = c * ap - sn * aq;
-        Am[r][q] = sn * ap + c * aq;
-        double zp = Zm[r][p], zq = Zm[r][q];
-        Zm[r][p] = c * zp - sn * zq;
-        Zm[r][q] = sn * zp + c * zq;
-      }
-      __syncthreads();
-      // rows: A <- J^T A
-      for (int item = tid; item < (mp / 2) * LEAF; item += blockDim.x) {
-        int pi = item / LEAF, col = item % LEAF;
-        int p = pr[pi][0], q = pr[pi][1];
-        if (q >= m || col >= m) continue;
-        double c = cs[pi][0], sn = cs[pi][1];
-        double ap = Am[p][col], aq = Am[q][col];
-        Am[p][col] = c * ap - sn * aq;
-        Am[q][col] = sn * ap + c * aq;
-      }
-      __syncthreads();
-      // the rotation annihilates a_pq exactly in exact arithmetic
-      if (tid < mp / 2 && pr[tid][1] < m && cs[tid][1] != 0.0) {
-        Am[pr[tid][0]][pr[tid][1]] = 0.0;
-        Am[pr[tid][1]][pr[tid][0]] = 0.0;
+      {
+        const int i = tid / NP, j = tid % NP;
+        if (i < mp / 2 && j < mp / 2) {
+          const int pi = pr[i][0], qi = pr[i][1], pj = pr[j][0], qj = pr[j][1];
+          const double ci = cs[i][0], si = cs[i][1], cj = cs[j][0], sj = cs[j][1];
+          const double app = Am[pi][pj], apq = Am[pi][qj], aqp = Am[qi][pj], aqq = Am[qi][qj];
+          // columns, then rows; the dummy's row and column are zero and stay so
+          const double bpp = cj * app - sj * apq, bpq = sj * app + cj * apq;
+          const double bqp = cj * aqp - sj * aqq, bqq = sj * aqp + cj * aqq;
+          const bool own = i == j && si != 0.0;  // a_pq vanishes in exact arithmetic
+          Am[pi][pj] = ci * bpp - si * bqp;
+          Am[pi][qj] = own ? 0.0 : ci * bpq - si * bqq;
+          Am[qi][pj] = own ? 0.0 : si * bpp + ci * bqp;
+          Am[qi][qj] = si * bpq + ci * bqq;
+          // rows i and i + NP of Z
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const int r = i + h * (mp / 2);
+            const double zp = Zm[r][pj], zq = Zm[r][qj];
+            Zm[r][pj] = cj * zp - sj * zq;
+            Zm[r][qj] = sj * zp + cj * zq;
+          }
+        }
       }
       __syncthreads();
     }
     if (sweep == max_sweeps - 1 && tid == 0) atomicOr(err, 2);
-    __syncthreads();
   }
-  // sort ascending (insertion sort of m values)
-  if (tid == 0) {
+  // ascending order: the rank of each value (ties by index)
+  __syncthreads();
+  if (tid < m) {
+    const double v = Am[tid][tid];
+    int rank = 0;
     for (int c = 0; c < m; ++c) {
-      s_val[c] = Am[c][c];
-      s_idx[c] = c;
+      const double o = Am[c][c];
+      rank += (o < v || (o == v && c < tid)) ? 1 : 0;
     }
-    for (int c = 1; c < m; ++c) {
-      double v = s_val[c];
-      int ix = s_idx[c], p = c - 1;
-      while (p >= 0 && s_val[p] > v) {
-        s_val[p + 1] = s_val[p];
-        s_idx[p + 1] = s_idx[p];
-        --p;
-      }
-      s_val[p + 1] = v;
-      s_idx[p + 1] = ix;
-    }
+    s_idx[rank] = tid;
+    w[s0 + rank] = v;
   }
   __syncthreads();
-  for (int q = tid; q < m * m; q += blockDim.x) {
+  for (int q = tid; q < m * m; q += 256) {
     int r = q % m, c = q / m;
     Z[(s0 + r) + (long long)(s0 + c) * ldz] = Zm[r][s_idx[c]];
   }
-  for (int c = tid; c < m; c += blockDim.x) w[s0 + c] = s_val[c];
 }
 
 struct DcWork {
@@ -882,12 +898,17 @@ __global__ void dc_assemble_kernel(const Node* nodes, DcWork wk, const double* O
 // The Gram matrices and T factors are stored per pair of blocks (2 NBB x
 // 2 NBB, leading dimension ldg = ldt = 2 NBB): block b is the diagonal
 // sub-block b % 2 of pair b / 2.
-__global__ void __launch_bounds__(NBB) larft_kernel(const double* Gall, long long ldg,
-                                                    const double* tau_all, int nref,
-                                                    double* Tall, long long ldt) {
+// What bounds it: the chain of NBB columns.  Four lanes share a row's sum, four
+// terms in flight each: order 72, 57 -> 37 us with a thread per row; twelve
+// blocks at 1453, 136 -> 93.
+constexpr int LARFT_LANES = 4;
+__global__ void __launch_bounds__(NBB * LARFT_LANES) larft_kernel(const double* Gall,
+                                                                  long long ldg,
+                                                                  const double* tau_all, int nref,
+                                                                  double* Tall, long long ldt) {
   extern __shared__ double smem_t[];
   double(*S)[NBB + 1] = reinterpret_cast<double(*)[NBB + 1]>(smem_t);
-  const int r = threadIdx.x;
+  const int tid = threadIdx.x, r = tid / LARFT_LANES, part = tid % LARFT_LANES;
   const int j0 = blockIdx.x * NBB, jb = min(NBB, nref - j0);
   if (jb <= 0) return;
   const int pr = blockIdx.x >> 1, h = blockIdx.x & 1;
@@ -895,23 +916,37 @@ __global__ void __launch_bounds__(NBB) larft_kernel(const double* Gall, long lon
   const double* tau = tau_all + j0;
   double* T = Tall + (size_t)pr * 2 * NBB * ldt + (size_t)h * NBB * (ldt + 1);
   // S[c][r] = G(r, c) for r < c (lower triangle); the upper triangle holds T
-  for (int c = 0; c < jb; ++c) {
-    if (r <= c) S[r][c] = 0.0;                          // T part: upper triangle
-    else S[r][c] = G[c + (long long)r * ldg];           // G(c, r), c < r: lower triangle
+  for (int q = tid; q < jb * NBB; q += NBB * LARFT_LANES) {
+    const int c = q % NBB, rr = q / NBB;
+    if (c < jb) S[rr][c] = rr <= c ? 0.0 : G[c + (long long)rr * ldg];
   }
   __syncthreads();
   for (int i = 0; i < jb; ++i) {
     const double ti = tau[i];
-    double s = 0.0;
-    if (r < i)
-      for (int c = r; c < i; ++c) s += S[r][c] * S[i][c];
-    __syncthreads();
-    if (r < i) S[r][i] = -ti * s;
-    if (r == i) S[i][i] = ti;
+    double s[4] = {0.0, 0.0, 0.0, 0.0};
+    if (r < i) {
+      int c = r + part;
+      for (; c + 3 * LARFT_LANES < i; c += 4 * LARFT_LANES)
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          s[u] = fma(S[r][c + u * LARFT_LANES], S[i][c + u * LARFT_LANES], s[u]);
+#pragma unroll
+      for (int u = 0; u < 3; ++u)
+        if (c + u * LARFT_LANES < i)
+          s[u] = fma(S[r][c + u * LARFT_LANES], S[i][c + u * LARFT_LANES], s[u]);
+    }
+    double sum = (s[0] + s[1]) + (s[2] + s[3]);
+    sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+    sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+    // column i of T is read from the next column on only
+    if (part == 0 && r < i) S[r][i] = -ti * sum;
+    if (part == 0 && r == i) S[i][i] = ti;
     __syncthreads();
   }
-  for (int c = 0; c < jb; ++c)
-    if (r < jb) T[r + (long long)c * ldt] = (r <= c) ? S[r][c] : 0.0;
+  for (int q = tid; q < jb * NBB; q += NBB * LARFT_LANES) {
+    const int rr = q % NBB, c = q / NBB;
+    if (rr < jb) T[rr + (long long)c * ldt] = rr <= c ? S[rr][c] : 0.0;
+  }
 }
 
 }  // namespace
@@ -1236,7 +1271,7 @@ int eigen_dc(imcom_ctx* ctx, const DMat& A, DMat& Wout, double* wout) {
   if (!splits.empty()) {
     IMC_CUDA(cudaMemcpyAsync(dsplit, splits.data(), splits.size() * 4, cudaMemcpyHostToDevice,
                              ctx->stream));
-    tear_kernel<<<1, 1, 0, ctx->stream>>>(dt, e, dsplit, (int)splits.size());
+    tear_kernel<<<(unsigned)(splits.size() + 255) / 256, 256, 0, ctx->stream>>>(dt, e, dsplit, (int)splits.size());
     IMC_LAUNCH();
   }
   // Z buffers: ZA = Wout, ZB = Aw (the A copy is no longer needed after sytrd...
@@ -1372,7 +1407,7 @@ int eigen_dc(imcom_ctx* ctx, const DMat& A, DMat& Wout, double* wout) {
                   Gb + (size_t)pi * NB2 * NB2, NB2));
   }
   IMC_CUDA(cudaMemsetAsync(Tb, 0, (size_t)npair * NB2 * NB2 * sizeof(double), ctx->stream));
-  larft_kernel<<<nblk, NBB, LARFT_SMEM, ctx->stream>>>(Gb, NB2, tau, nref, Tb, NB2);
+  larft_kernel<<<nblk, NBB * LARFT_LANES, LARFT_SMEM, ctx->stream>>>(Gb, NB2, tau, nref, Tb, NB2);
   IMC_LAUNCH();
   for (int pi = 0; pi < npair; ++pi) {
     const int j0 = pi * NB2, jb = std::min(NB2, nref - j0);
