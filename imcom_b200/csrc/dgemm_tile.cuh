@@ -233,5 +233,111 @@ dgemm_persist_kernel(long long M, long long N, long long K, double alpha,
   }
 }
 
+// Products whose 128 x 128 tiles leave most SMs idle: 32 x 32 tiles of 4 warps
+// (2 x 2, a warp 16 x 16), three stages of 32 deep, up to four CTAs per SM.  The sum
+// over k runs in the same order as above, so without split-K the results are the
+// same to the bit.
+constexpr int SBM = 32, SSTRIDE = SBM + 4, STHREADS = 128, SSTAGES = 3;
+static_assert(BK == SBM, "either order of a tile has 32 lines of 32");
+constexpr int SSTAGE_DBL = 2 * SBM * SSTRIDE;
+constexpr size_t SSMEM_BYTES = (size_t)SSTAGES * SSTAGE_DBL * sizeof(double);
+
+// Microseconds of a product in small tiles (a step of 32 deep costs 0.7 us with
+// one CTA on an SM, 0.42 per CTA with more) and in large ones (per step of 32, waves
+// x depth).
+inline double small_tiles_us(long long tiles, long long K, int sms) {
+  const double per = 0.42 * (double)((tiles + sms - 1) / sms);
+  return 2.5 + (double)((K + BK - 1) / BK) * (per > 0.7 ? per : 0.7);
+}
+inline double large_tiles_us(double steps) { return 3.0 + 0.14 * BK * steps; }
+
+template <bool AK, bool BKC, int VEC>
+__device__ __forceinline__ void dgemm_small_tile(int M, int N, int K, double alpha,
+                                                 const double* __restrict__ A, long long lda,
+                                                 const double* __restrict__ B, long long ldb,
+                                                 double beta, double* __restrict__ C,
+                                                 long long ldc, int m0, int n0) {
+  extern __shared__ __align__(16) double smem[];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int wm = (warp & 1) * 16, wn = (warp >> 1) * 16, g = lane >> 2, t = lane & 3;
+  constexpr int PER = SBM / VEC, LINES = STHREADS / PER;
+  const int li = tid / PER, lo = tid % PER * VEC;
+  // lines of a tile: rows of k if k is contiguous, else k of rows
+  auto load = [&](double* S, const double* P, long long ld, bool kc, int r0, int R, int k0) {
+#pragma unroll
+    for (int i = li; i < SBM; i += LINES) {
+      const int r = r0 + (kc ? i : lo), k = k0 + (kc ? lo : i);
+      const int v = kc ? (r < R ? min(VEC, K - k) : 0) : (k < K ? min(VEC, R - r) : 0);
+      cp_async(S + i * SSTRIDE + lo, v > 0 ? (kc ? P + k + r * ld : P + r + k * ld) : P,
+               8 * max(v, 0), VEC);
+    }
+  };
+  const int nk = (K + BK - 1) / BK;
+  double acc[2][4] = {};
+#pragma unroll
+  for (int s = 0; s < SSTAGES - 1; ++s) {
+    if (s < nk) {
+      load(smem + s * SSTAGE_DBL, A, lda, AK, m0, M, s * BK);
+      load(smem + s * SSTAGE_DBL + SSTAGE_DBL / 2, B, ldb, BKC, n0, N, s * BK);
+    }
+    cp_commit();
+  }
+  for (int kt = 0; kt < nk; ++kt) {
+    cp_wait<SSTAGES - 2>();
+    __syncthreads();
+    const int nx = kt + SSTAGES - 1;
+    if (nx < nk) {
+      double* Sn = smem + nx % SSTAGES * SSTAGE_DBL;
+      load(Sn, A, lda, AK, m0, M, nx * BK);
+      load(Sn + SSTAGE_DBL / 2, B, ldb, BKC, n0, N, nx * BK);
+    }
+    cp_commit();
+    const double* As = smem + kt % SSTAGES * SSTAGE_DBL;
+    const double* Bs = As + SSTAGE_DBL / 2;
+#pragma unroll
+    for (int kk = 0; kk < BK; kk += 4) {
+      const int k = kk + t;
+      const double a0 = AK ? As[(wm + g) * SSTRIDE + k] : As[k * SSTRIDE + wm + g];
+      const double a1 = AK ? As[(wm + g + 8) * SSTRIDE + k] : As[k * SSTRIDE + wm + g + 8];
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        const int nc = wn + 8 * j + g;
+        const double b = BKC ? Bs[nc * SSTRIDE + k] : Bs[k * SSTRIDE + nc];
+        asm volatile(
+            "mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5}, {%6}, "
+            "{%0,%1,%2,%3};\n"
+            : "+d"(acc[j][0]), "+d"(acc[j][1]), "+d"(acc[j][2]), "+d"(acc[j][3])
+            : "d"(a0), "d"(a1), "d"(b));
+      }
+    }
+  }
+  cp_wait<0>();
+#pragma unroll
+  for (int j = 0; j < 2; ++j)
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const int row = m0 + wm + g + ((r >> 1) ? 8 : 0), col = n0 + wn + 8 * j + 2 * t + (r & 1);
+      if (row < M && col < N) {
+        double* c = C + row + col * ldc;
+        *c = beta != 0.0 ? fma(beta, *c, alpha * acc[j][r]) : alpha * acc[j][r];
+      }
+    }
+}
+
+// CTA b takes tiles b, b + gridDim.x, ... (a context on a share of the SMs has fewer
+// CTAs than tiles).
+template <bool AK, bool BKC, int VEC>
+__global__ void __launch_bounds__(STHREADS)
+dgemm_small_kernel(int M, int N, int K, double alpha, const double* __restrict__ A, long long lda,
+                   const double* __restrict__ B, long long ldb, double beta,
+                   double* __restrict__ C, long long ldc) {
+  const int gm = (M + SBM - 1) / SBM, total = gm * ((N + SBM - 1) / SBM);
+  for (int tile = blockIdx.x; tile < total; tile += gridDim.x) {
+    __syncthreads();  // every warp is done with the previous tile's shared stages
+    dgemm_small_tile<AK, BKC, VEC>(M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, tile % gm * SBM,
+                                   tile / gm * SBM);
+  }
+}
+
 }  // namespace gemm
 }  // namespace imcom

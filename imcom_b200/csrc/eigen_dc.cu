@@ -848,6 +848,24 @@ dc_gemm_kernel(const Node* nodes, const int* kcnt, const double* G, const double
   }
 }
 
+// The same in small tiles (dgemm_tile.cuh), for levels that leave most SMs idle.
+template <int VEC>
+__global__ void __launch_bounds__(gemm::STHREADS)
+dc_gemm_small_kernel(const Node* nodes, const int* kcnt, const double* G, const double* U,
+                     double* OUT, long long ld, int tiles, int nn) {
+  const int total = tiles * tiles * nn;
+  for (int b = blockIdx.x; b < total; b += gridDim.x) {
+    const int z = b / (tiles * tiles), xy = b - z * tiles * tiles;
+    const Node nd = nodes[z];
+    const int k = kcnt[z], m0 = xy % tiles * gemm::SBM, n0 = xy / tiles * gemm::SBM;
+    if (m0 >= nd.nm || n0 >= k) continue;  // uniform over the CTA
+    __syncthreads();  // every warp is done with the previous tile's shared stages
+    const size_t off = (size_t)nd.s + (size_t)nd.s * ld;
+    gemm::dgemm_small_tile<false, true, VEC>(nd.nm, k, k, 1.0, G + off, ld, U + off, ld, 0.0,
+                                             OUT + off, ld, m0, n0);
+  }
+}
+
 // Rank of each new eigenvalue within its node (stable, O(nm) per element).
 // One warp per element: the lanes split the comparisons and add their counts.
 __global__ void dc_rank_kernel(const Node* nodes, DcWork wk) {
@@ -1351,7 +1369,19 @@ int eigen_dc(imcom_ctx* ctx, const DMat& A, DMat& Wout, double* wout) {
       const unsigned total = tiles * tiles * (unsigned)nn_;
       // a context on a share of the SMs: at most one CTA per SM of its share
       const unsigned gd = ctx->sm_share > 0 ? std::min(total, (unsigned)sm_count(ctx)) : total;
-      if (even) {
+      const long long ts = (maxnm + gemm::SBM - 1) / gemm::SBM, small = ts * ts * nn_;
+      const int sms = sm_count(ctx);
+      // as dgemm's rule; the six levels of order 1453 353 -> 210 us, of 72 27 -> 9
+      if (total < (unsigned)sms &&
+          gemm::small_tiles_us(small, maxnm, sms) <
+              0.9 * gemm::large_tiles_us((maxnm + gemm::BK - 1) / gemm::BK)) {
+        auto k = even ? dc_gemm_small_kernel<2> : dc_gemm_small_kernel<1>;
+        IMC_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)gemm::SSMEM_BYTES));
+        const unsigned gs = (unsigned)(ctx->sm_share > 0 ? std::min<long long>(small, 4LL * sms) : small);
+        k<<<gs, gemm::STHREADS, gemm::SSMEM_BYTES, ctx->stream>>>(dnodes, wk.kcnt, Gm, Ub, OUT, UO.ld,
+                                                                  (int)ts, nn_);
+      } else if (even) {
         IMC_CUDA(cudaFuncSetAttribute(dc_gemm_kernel<2>,
                                       cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)gemm::SMEM_BYTES));
