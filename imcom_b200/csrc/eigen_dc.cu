@@ -42,7 +42,8 @@ constexpr int NB = TRD_NB;        // tridiagonalisation panel width
 constexpr int LEAF = 32;          // largest leaf of the divide-and-conquer tree
 constexpr int NBB = 128;          // reflectors per back-transformation block
 constexpr double EPS = 1.1102230246251565e-16;
-constexpr size_t LARFT_SMEM = (size_t)NBB * (NBB + 1) * sizeof(double);
+// the T factor's tile and the joins' product
+constexpr size_t LARFT_SMEM = ((size_t)NBB * (NBB + 1) + (NBB - 32) * 33) * sizeof(double);
 
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
@@ -916,10 +917,12 @@ __global__ void dc_assemble_kernel(const Node* nodes, DcWork wk, const double* O
 // The Gram matrices and T factors are stored per pair of blocks (2 NBB x
 // 2 NBB, leading dimension ldg = ldt = 2 NBB): block b is the diagonal
 // sub-block b % 2 of pair b / 2.
-// What bounds it: the chain of NBB columns.  Four lanes share a row's sum, four
-// terms in flight each: order 72, 57 -> 37 us with a thread per row; twelve
-// blocks at 1453, 136 -> 93.
-constexpr int LARFT_LANES = 4;
+// What bounds it: the chain of columns, so only blocks of LARFT_B run it (four
+// lanes per row, all blocks of the CTA at once); block b then joins the ones before it
+// by T(0:i0, b) = -T(0:i0, 0:i0) (G(0:i0, b) T(b, b)), a lane per column, a warp per
+// six rows.  Order 72: 57 us with a thread per row, 32 now; twelve CTAs at 1453, 136
+// -> 52 (the whole chain with four lanes per row: 37 and 93).
+constexpr int LARFT_LANES = 4, LARFT_B = 32;
 __global__ void __launch_bounds__(NBB * LARFT_LANES) larft_kernel(const double* Gall,
                                                                   long long ldg,
                                                                   const double* tau_all, int nref,
@@ -939,26 +942,57 @@ __global__ void __launch_bounds__(NBB * LARFT_LANES) larft_kernel(const double* 
     if (c < jb) S[rr][c] = rr <= c ? 0.0 : G[c + (long long)rr * ldg];
   }
   __syncthreads();
-  for (int i = 0; i < jb; ++i) {
-    const double ti = tau[i];
-    double s[4] = {0.0, 0.0, 0.0, 0.0};
-    if (r < i) {
-      int c = r + part;
-      for (; c + 3 * LARFT_LANES < i; c += 4 * LARFT_LANES)
+  {
+    const int i0 = r / LARFT_B * LARFT_B, rl = r % LARFT_B, ib = jb - i0;
+#pragma unroll 1
+    for (int i = 0; i < LARFT_B; ++i) {
+      double s = 0.0;
+      if (i < ib && rl < i)
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
-          s[u] = fma(S[r][c + u * LARFT_LANES], S[i][c + u * LARFT_LANES], s[u]);
-#pragma unroll
-      for (int u = 0; u < 3; ++u)
-        if (c + u * LARFT_LANES < i)
-          s[u] = fma(S[r][c + u * LARFT_LANES], S[i][c + u * LARFT_LANES], s[u]);
+        for (int u = 0; u < LARFT_B / LARFT_LANES; ++u) {
+          const int c = rl + part + u * LARFT_LANES;
+          if (c < i) s = fma(S[r][i0 + c], S[i0 + i][i0 + c], s);
+        }
+      s += __shfl_xor_sync(0xffffffffu, s, 1);
+      s += __shfl_xor_sync(0xffffffffu, s, 2);
+      // column i of T is read from the next column on only
+      if (part == 0 && i < ib && rl <= i) S[r][i0 + i] = rl == i ? tau[r] : -tau[i0 + i] * s;
+      __syncthreads();
     }
-    double sum = (s[0] + s[1]) + (s[2] + s[3]);
-    sum += __shfl_xor_sync(0xffffffffu, sum, 1);
-    sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-    // column i of T is read from the next column on only
-    if (part == 0 && r < i) S[r][i] = -ti * sum;
-    if (part == 0 && r == i) S[i][i] = ti;
+  }
+  constexpr int NW = NBB * LARFT_LANES / 32, RW = (NBB - LARFT_B) / NW;
+  static_assert(LARFT_B == 32 && RW * NW == NBB - LARFT_B, "a lane per column of a block");
+  double(*X)[LARFT_B + 1] = reinterpret_cast<double(*)[LARFT_B + 1]>(smem_t + NBB * (NBB + 1));
+  const int j = tid % 32, w = tid / 32;
+  for (int i0 = LARFT_B; i0 < jb; i0 += LARFT_B) {
+    const int ib = min(LARFT_B, jb - i0);
+    double acc[RW];
+#pragma unroll
+    for (int q = 0; q < RW; ++q) acc[q] = 0.0;
+#pragma unroll 4
+    for (int c = 0; c < ib; ++c) {
+      const double t = (j < ib && c <= j) ? S[i0 + c][i0 + j] : 0.0;
+#pragma unroll
+      for (int q = 0; q < RW; ++q)
+        if (w + NW * q < i0) acc[q] = fma(S[i0 + c][w + NW * q], t, acc[q]);
+    }
+#pragma unroll
+    for (int q = 0; q < RW; ++q) {
+      if (w + NW * q < i0) X[w + NW * q][j] = acc[q];
+      acc[q] = 0.0;
+    }
+    __syncthreads();
+#pragma unroll 4
+    for (int c = 0; c < i0; ++c) {
+      const double x = X[c][j];
+#pragma unroll
+      for (int q = 0; q < RW; ++q)
+        if (w + NW * q <= c) acc[q] = fma(S[w + NW * q][c], x, acc[q]);
+    }
+    if (j < ib)
+#pragma unroll
+      for (int q = 0; q < RW; ++q)
+        if (w + NW * q < i0) S[w + NW * q][i0 + j] = -acc[q];
     __syncthreads();
   }
   for (int q = tid; q < jb * NBB; q += NBB * LARFT_LANES) {
