@@ -646,22 +646,27 @@ __global__ void __launch_bounds__(LB_WARPS * 32, 7) learned_fused_kernel(BisectA
 // term with the target held fixed (it fits the log of the first head's error).
 //
 // One cooperative launch runs an epoch.  A CTA takes tiles of 32 samples of
-// each batch, sums its gradients in registers and adds them to the batch's
-// gradient with one atomic per parameter; past the grid barrier every CTA reads
-// the whole gradient and takes the same Adam step on its own copy of the
-// parameters: fp32 parameters and moments in registers, the rounded weights in
-// shared memory.  Three gradient buffers in turn leave one to clear.
+// each batch and leaves every tile's sums in a row of global memory.  Past a grid
+// barrier CTA q adds up its slice of the parameters, tile by tile in ascending
+// order, takes the Adam step on that slice (fp32 parameters and moments in
+// registers) and writes the new parameters; past a second barrier every CTA
+// rounds them into its shared memory.  So a result depends neither on timing nor
+// on the grid.
 // What bounds it: shared-memory reads of the 64 x 64 layer (about 6000 cycles a
-// tile), the barrier and the chain of small layers.  A step of 512 samples: 29
-// us as three launches (clear, gradient, Adam) with layer 2 reading its weights
-// 64 floats apart, 13 now.  Tiles of eight samples are as fast at 512 samples, but
-// add up in other partial sums.
+// tile), the barriers and the chain of small layers.  20000 samples, two epochs of 40
+// batches of 512: 2557 us as three launches a batch (clear, gradient, Adam), 1240 with
+// one atomic per parameter and tile and Adam on every CTA's own copy (in arrival
+// order, which Adam and the rounded weights amplify to 1e-3 of the parameters), 1199
+// now.  Tiles of eight samples are as fast at 512 samples, but add up in other
+// partial sums.
 // ---------------------------------------------------------------------------
 constexpr int TB = 32;              // samples per tile
 constexpr int TRAIN_THREADS = 512;  // thread: unit u = tid % 64 of RPT rows tid / 64 + RG i
 constexpr int RG = TRAIN_THREADS / NH, RPT = TB / RG;
-constexpr int PPT = (NPARAM + TRAIN_THREADS - 1) / TRAIN_THREADS;  // parameters per thread
-constexpr int GSTRIDE = (NPARAM + 3) / 4 * 4;                      // a gradient buffer
+constexpr int NSUM = NPARAM + 1;                                // a tile's sums: gradient, loss
+constexpr int PPT = (NSUM + TRAIN_THREADS - 1) / TRAIN_THREADS;  // of them per thread
+constexpr int GSTRIDE = (NSUM + 3) / 4 * 4;                     // a tile's row
+constexpr int TRAIN_ROWS = 1024;  // rows at most (21 MB); a batch of more tiles takes several rounds
 
 struct TrainArgs {
   float* params;  // packed
@@ -670,7 +675,9 @@ struct TrainArgs {
   const float* target;
   const int* idx;     // order of the samples, or null
   int nsamples, batch;
-  float* grad;        // GSTRIDE floats, zero; three of them when training
+  float* part;        // rows of GSTRIDE floats
+  int rows;           // a multiple of the grid
+  float* grad;        // the gradient (not when training)
   float* loss;
   float *m1, *m2;     // Adam moments
   const float2* c12;  // per step: 1 - b1^step, 1 - b2^step
@@ -689,11 +696,14 @@ __global__ void __launch_bounds__(TRAIN_THREADS, 1) mlp_train_kernel(TrainArgs a
   // activations, and the gradients before the ReLUs (layer 1's in place of H2)
   __shared__ __align__(16) float H1[TB][NH], D2[TB][NH];
   __shared__ float H2[TB][NH + 1];
-  __shared__ float DO[TB][NO];
+  __shared__ float DO[TB][NO], sl[TB];
   __shared__ int s_stop;
   const int tid = threadIdx.x;
   const int u = tid % NH, rg = tid / NH;
   const int G = gridDim.x, steps = (a.nsamples + a.batch - 1) / a.batch;
+  // this CTA's slice of the sums; parameters and moments of its gradient's part, the
+  // epoch's loss in the loss's place
+  const int q0 = NSUM * (int)blockIdx.x / G, q1 = NSUM * ((int)blockIdx.x + 1) / G;
   float p[PPT], m1[PPT], m2[PPT];
   auto store_weight = [&](int q, float v) {
     if (q < OFF_B1) sW1[q % NF][q / NF] = bf16r(v);
@@ -703,21 +713,28 @@ __global__ void __launch_bounds__(TRAIN_THREADS, 1) mlp_train_kernel(TrainArgs a
     else if (q < OFF_B3) sW3[(q - OFF_W3) / NH][(q - OFF_W3) % NH] = bf16r(v);
     else sb3[q - OFF_B3] = v;
   };
+  auto load_weights = [&]() {
+    float v[PPT];
+#pragma unroll
+    for (int i = 0; i < PPT; ++i) {
+      const int q = tid + TRAIN_THREADS * i;
+      v[i] = q < NPARAM ? __ldcg(a.params + q) : 0.0f;
+    }
+#pragma unroll
+    for (int i = 0; i < PPT; ++i)
+      if (tid + TRAIN_THREADS * i < NPARAM) store_weight(tid + TRAIN_THREADS * i, v[i]);
+  };
+  load_weights();
 #pragma unroll
   for (int i = 0; i < PPT; ++i) {
-    const int q = tid + TRAIN_THREADS * i;
+    const int q = q0 + tid + TRAIN_THREADS * i;
     p[i] = m1[i] = m2[i] = 0.0f;
-    if (q < NPARAM) {
-      p[i] = a.params[q];
-      if (TRAIN) {
-        m1[i] = a.m1[q];
-        m2[i] = a.m2[q];
-      }
+    if (TRAIN && q < min(q1, NPARAM)) {
+      p[i] = __ldcg(a.params + q);
+      m1[i] = a.m1[q];
+      m2[i] = a.m2[q];
     }
   }
-#pragma unroll
-  for (int i = 0; i < PPT; ++i)
-    if (tid + TRAIN_THREADS * i < NPARAM) store_weight(tid + TRAIN_THREADS * i, p[i]);
   if (tid == 0) s_stop = 0;
 
   static_assert(RG == NF / 2 + 2, "row groups: six of dW1, db1, db2");
@@ -759,151 +776,18 @@ __global__ void __launch_bounds__(TRAIN_THREADS, 1) mlp_train_kernel(TrainArgs a
   fetch_index();
   fetch_data();
 
-  const int tu = tid / 32, tv = tid % 32;  // dW2: units 4 tu .., inputs tv and tv + 32
-  float lsum = 0.0f;
-  for (int step = 0; step < steps; ++step) {
-    const int nb = min(a.batch, a.nsamples - step * a.batch);
-    float gW2[4][2] = {}, gW1[2] = {}, gb = 0.0f, gW3 = 0.0f;
-    for (int tile = blockIdx.x; tile * TB < nb; tile += G) {
-      if (lt >= 0 && lt < FEATS) X0[lrow][lk] = x_next;
-      else if (lt >= FEATS && lt < FEATS + TB) sy[lrow] = x_next;
-      __syncthreads();
-      if (tile + G < (nb + TB - 1) / TB) fetch_data();
-      // layer 1
-      float h1[RPT];
-#pragma unroll
-      for (int i = 0; i < RPT; ++i) {
-        float s = sb1[u];
-#pragma unroll
-        for (int k = 0; k < NF; ++k) s = fmaf(sW1[k][u], X0[rg + RG * i][k], s);
-        h1[i] = bf16r(fmaxf(s, 0.0f));
-        H1[rg + RG * i][u] = h1[i];
-      }
-      __syncthreads();
-      // layer 2
-      float h2[RPT];
-#pragma unroll
-      for (int i = 0; i < RPT; ++i) h2[i] = sb2[u];
-#pragma unroll 4
-      for (int v = 0; v < NH; v += 4) {
-        const float w0 = sW2[v][u], w1 = sW2[v + 1][u], w2 = sW2[v + 2][u], w3 = sW2[v + 3][u];
-#pragma unroll
-        for (int i = 0; i < RPT; ++i) {
-          const float4 h = *(const float4*)&H1[rg + RG * i][v];
-          h2[i] = fmaf(w3, h.w, fmaf(w2, h.z, fmaf(w1, h.y, fmaf(w0, h.x, h2[i]))));
-        }
-      }
-#pragma unroll
-      for (int i = 0; i < RPT; ++i) {
-        h2[i] = bf16r(fmaxf(h2[i], 0.0f));
-        H2[rg + RG * i][u] = h2[i];
-      }
-      __syncthreads();
-      // output, loss and d loss / d output: a lane per sample and output
-      if (tid < NO * TB) {
-        const int r = tid / NO, j = tid % NO;
-        float o = sb3[j];
-#pragma unroll 16
-        for (int v = 0; v < NH; ++v) o = fmaf(sW3[j][v], H2[r][v], o);
-        const float o1 = __shfl_down_sync(0xffffffffu, o, 1);
-        if (j == 0) {
-          float d0 = 0.0f, d1 = 0.0f;
-          if (tile * TB + r < nb) {
-            const float e = o - sy[r];
-            const float ltar = logf(fabsf(e) + 0.01f);
-            const float e1 = o1 - ltar;
-            lsum += e * e + 0.25f * e1 * e1;
-            d0 = 2.0f * e;
-            d1 = 0.5f * e1;
-          }
-          DO[r][0] = d0;
-          DO[r][1] = d1;
-        }
-      }
-      __syncthreads();
-#pragma unroll
-      for (int i = 0; i < RPT; ++i) {
-        const int r = rg + RG * i;
-        const float g = DO[r][0] * sW3[0][u] + DO[r][1] * sW3[1][u];
-        D2[r][u] = h2[i] > 0.0f ? g : 0.0f;
-      }
-      if (tid < NO * NH) {
-#pragma unroll 8
-        for (int r = 0; r < TB; ++r) gW3 = fmaf(DO[r][rg], H2[r][u], gW3);
-      } else if (tid < NO * NH + NO) {
-#pragma unroll 8
-        for (int r = 0; r < TB; ++r) gW3 += DO[r][tid - NO * NH];
-      }
-      __syncthreads();
-      // dW2 = dH2^T H1, and db2
-#pragma unroll 4
-      for (int r = 0; r < TB; ++r) {
-        const float4 d = *(const float4*)&D2[r][4 * tu];
-        const float dd[4] = {d.x, d.y, d.z, d.w}, hh[2] = {H1[r][tv], H1[r][tv + 32]};
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-          for (int j = 0; j < 2; ++j) gW2[i][j] = fmaf(dd[i], hh[j], gW2[i][j]);
-      }
-      if (rg == RG - 1) {
-#pragma unroll 8
-        for (int r = 0; r < TB; ++r) gb += D2[r][u];
-      }
-      // dH1 = W2^T dH2 where the ReLU passes
-      float d1[RPT] = {};
-#pragma unroll 4
-      for (int v = 0; v < NH; v += 4) {
-        const float w0 = sW2[u][v], w1 = sW2[u][v + 1], w2 = sW2[u][v + 2], w3 = sW2[u][v + 3];
-#pragma unroll
-        for (int i = 0; i < RPT; ++i) {
-          const float4 d = *(const float4*)&D2[rg + RG * i][v];
-          d1[i] = fmaf(w3, d.w, fmaf(w2, d.z, fmaf(w1, d.y, fmaf(w0, d.x, d1[i]))));
-        }
-      }
-#pragma unroll
-      for (int i = 0; i < RPT; ++i) H2[rg + RG * i][u] = h1[i] > 0.0f ? d1[i] : 0.0f;
-      __syncthreads();
-      // dW1 = dH1^T X0, and db1
-      if (rg < NF / 2) {
-#pragma unroll 8
-        for (int r = 0; r < TB; ++r) {
-          const float d = H2[r][u];
-          gW1[0] = fmaf(d, X0[r][2 * rg], gW1[0]);
-          gW1[1] = fmaf(d, X0[r][2 * rg + 1], gW1[1]);
-        }
-      } else if (rg == NF / 2) {
-#pragma unroll 8
-        for (int r = 0; r < TB; ++r) gb += H2[r][u];
-      }
-      __syncthreads();
-    }
-    float* grad = a.grad + (TRAIN ? step % 3 : 0) * GSTRIDE;
-    if (blockIdx.x * TB < nb) {
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 2; ++j)
-          atomicAdd(grad + OFF_W2 + (4 * tu + i) * NH + tv + 32 * j, gW2[i][j]);
-      if (rg < NF / 2) {
-        atomicAdd(grad + OFF_W1 + u * NF + 2 * rg, gW1[0]);
-        atomicAdd(grad + OFF_W1 + u * NF + 2 * rg + 1, gW1[1]);
-      } else if (rg == NF / 2) {
-        atomicAdd(grad + OFF_B1 + u, gb);
-      } else {
-        atomicAdd(grad + OFF_B2 + u, gb);
-      }
-      if (tid < NO * NH + NO) atomicAdd(grad + OFF_W3 + tid, gW3);
-    }
-    if (!TRAIN) break;
-    // grid barrier; the next tile's data is on its way meanwhile
+  // Grid barrier: false if it timed out.  With `fetch` the next tile's data is on its
+  // way meanwhile.
+  unsigned want = 0;
+  auto grid_sync = [&](bool fetch) {
+    want += G;
     __syncthreads();
-    if (tid == 0) {
+    if (G > 1 && tid == 0) {
       __threadfence();
       atomicAdd(a.arrived, 1u);
     }
-    fetch_data();
-    if (tid == 0) {
-      const unsigned want = (unsigned)G * (step + 1);
+    if (fetch) fetch_data();
+    if (G > 1 && tid == 0) {
       long long it = 0;
       unsigned have;
       do {
@@ -916,39 +800,208 @@ __global__ void __launch_bounds__(TRAIN_THREADS, 1) mlp_train_kernel(TrainArgs a
       __threadfence();
     }
     __syncthreads();
-    if (s_stop) return;
-    const float2 c = a.c12[step];
-    const float inv = 1.0f / nb;
-    float gr[PPT];
+    return !s_stop;
+  };
+
+  const int tu = tid / 32, tv = tid % 32;  // dW2: units 4 tu .., inputs tv and tv + 32
+  for (int step = 0; step < steps; ++step) {
+    const int nb = min(a.batch, a.nsamples - step * a.batch), ntile = (nb + TB - 1) / TB;
+    float sum[PPT];
 #pragma unroll
-    for (int i = 0; i < PPT; ++i) {
-      const int q = tid + TRAIN_THREADS * i;
-      gr[i] = q < NPARAM ? __ldcg(grad + q) : 0.0f;
-    }
-    // the buffer of the step before last (read by every CTA before this barrier)
-    float* old = a.grad + (step + 2) % 3 * GSTRIDE;
-    for (int q = blockIdx.x * TRAIN_THREADS + tid; q < NPARAM; q += G * TRAIN_THREADS) old[q] = 0.0f;
+    for (int i = 0; i < PPT; ++i) sum[i] = q0 + tid + TRAIN_THREADS * i == NPARAM ? p[i] : 0.0f;
+    for (int first = 0; first < ntile; first += a.rows) {
+      const int last = min(ntile, first + a.rows), mine = first + blockIdx.x;
+      for (int tile = mine; tile < last; tile += G) {
+        float gW2[4][2] = {}, gW1[2] = {}, gb = 0.0f, gW3 = 0.0f;
+        if (lt >= 0 && lt < FEATS) X0[lrow][lk] = x_next;
+        else if (lt >= FEATS && lt < FEATS + TB) sy[lrow] = x_next;
+        __syncthreads();
+        if (tile + G < last) fetch_data();
+        // layer 1
+        float h1[RPT];
 #pragma unroll
-    for (int i = 0; i < PPT; ++i) {
-      const int q = tid + TRAIN_THREADS * i;
-      const float g = gr[i] * inv;
-      m1[i] = fmaf(a.b1, m1[i], (1.0f - a.b1) * g);
-      m2[i] = fmaf(a.b2, m2[i], (1.0f - a.b2) * g * g);
-      p[i] -= a.lr * (m1[i] / c.x) / (sqrtf(m2[i] / c.y) + 1e-8f);
-      if (q < NPARAM) store_weight(q, p[i]);
-    }
-    __syncthreads();
-  }
-  if (lsum != 0.0f) atomicAdd(a.loss, lsum);
-  if (TRAIN && blockIdx.x == 0) {
+        for (int i = 0; i < RPT; ++i) {
+          float s = sb1[u];
 #pragma unroll
-    for (int i = 0; i < PPT; ++i) {
-      const int q = tid + TRAIN_THREADS * i;
-      if (q < NPARAM) {
-        a.params[q] = p[i];
-        a.m1[q] = m1[i];
-        a.m2[q] = m2[i];
+          for (int k = 0; k < NF; ++k) s = fmaf(sW1[k][u], X0[rg + RG * i][k], s);
+          h1[i] = bf16r(fmaxf(s, 0.0f));
+          H1[rg + RG * i][u] = h1[i];
+        }
+        __syncthreads();
+        // layer 2
+        float h2[RPT];
+#pragma unroll
+        for (int i = 0; i < RPT; ++i) h2[i] = sb2[u];
+#pragma unroll 4
+        for (int v = 0; v < NH; v += 4) {
+          const float w0 = sW2[v][u], w1 = sW2[v + 1][u], w2 = sW2[v + 2][u], w3 = sW2[v + 3][u];
+#pragma unroll
+          for (int i = 0; i < RPT; ++i) {
+            const float4 h = *(const float4*)&H1[rg + RG * i][v];
+            h2[i] = fmaf(w3, h.w, fmaf(w2, h.z, fmaf(w1, h.y, fmaf(w0, h.x, h2[i]))));
+          }
+        }
+#pragma unroll
+        for (int i = 0; i < RPT; ++i) {
+          h2[i] = bf16r(fmaxf(h2[i], 0.0f));
+          H2[rg + RG * i][u] = h2[i];
+        }
+        __syncthreads();
+        // output, loss and d loss / d output: a lane per sample and output
+        if (tid < NO * TB) {
+          const int r = tid / NO, j = tid % NO;
+          float o = sb3[j];
+#pragma unroll 16
+          for (int v = 0; v < NH; ++v) o = fmaf(sW3[j][v], H2[r][v], o);
+          const float o1 = __shfl_down_sync(0xffffffffu, o, 1);
+          if (j == 0) {
+            float d0 = 0.0f, d1 = 0.0f, l = 0.0f;
+            if (tile * TB + r < nb) {
+              const float e = o - sy[r];
+              const float ltar = logf(fabsf(e) + 0.01f);
+              const float e1 = o1 - ltar;
+              l = e * e + 0.25f * e1 * e1;
+              d0 = 2.0f * e;
+              d1 = 0.5f * e1;
+            }
+            DO[r][0] = d0;
+            DO[r][1] = d1;
+            sl[r] = l;
+          }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < RPT; ++i) {
+          const int r = rg + RG * i;
+          const float g = DO[r][0] * sW3[0][u] + DO[r][1] * sW3[1][u];
+          D2[r][u] = h2[i] > 0.0f ? g : 0.0f;
+        }
+        if (tid < NO * NH) {
+#pragma unroll 8
+          for (int r = 0; r < TB; ++r) gW3 = fmaf(DO[r][rg], H2[r][u], gW3);
+        } else if (tid < NO * NH + NO) {
+#pragma unroll 8
+          for (int r = 0; r < TB; ++r) gW3 += DO[r][tid - NO * NH];
+        }
+        __syncthreads();
+        // dW2 = dH2^T H1, and db2
+#pragma unroll 4
+        for (int r = 0; r < TB; ++r) {
+          const float4 d = *(const float4*)&D2[r][4 * tu];
+          const float dd[4] = {d.x, d.y, d.z, d.w}, hh[2] = {H1[r][tv], H1[r][tv + 32]};
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 2; ++j) gW2[i][j] = fmaf(dd[i], hh[j], gW2[i][j]);
+        }
+        if (rg == RG - 1) {
+#pragma unroll 8
+          for (int r = 0; r < TB; ++r) gb += D2[r][u];
+        }
+        // dH1 = W2^T dH2 where the ReLU passes
+        float d1[RPT] = {};
+#pragma unroll 4
+        for (int v = 0; v < NH; v += 4) {
+          const float w0 = sW2[u][v], w1 = sW2[u][v + 1], w2 = sW2[u][v + 2], w3 = sW2[u][v + 3];
+#pragma unroll
+          for (int i = 0; i < RPT; ++i) {
+            const float4 d = *(const float4*)&D2[rg + RG * i][v];
+            d1[i] = fmaf(w3, d.w, fmaf(w2, d.z, fmaf(w1, d.y, fmaf(w0, d.x, d1[i]))));
+          }
+        }
+#pragma unroll
+        for (int i = 0; i < RPT; ++i) H2[rg + RG * i][u] = h1[i] > 0.0f ? d1[i] : 0.0f;
+        __syncthreads();
+        // dW1 = dH1^T X0, and db1
+        if (rg < NF / 2) {
+#pragma unroll 8
+          for (int r = 0; r < TB; ++r) {
+            const float d = H2[r][u];
+            gW1[0] = fmaf(d, X0[r][2 * rg], gW1[0]);
+            gW1[1] = fmaf(d, X0[r][2 * rg + 1], gW1[1]);
+          }
+        } else if (rg == NF / 2) {
+#pragma unroll 8
+          for (int r = 0; r < TB; ++r) gb += H2[r][u];
+        }
+        // the tile's row; its loss by halves
+        float* row = a.part + (size_t)(tile - first) * GSTRIDE;
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int j = 0; j < 2; ++j) row[OFF_W2 + (4 * tu + i) * NH + tv + 32 * j] = gW2[i][j];
+        if (rg < NF / 2) {
+          row[OFF_W1 + u * NF + 2 * rg] = gW1[0];
+          row[OFF_W1 + u * NF + 2 * rg + 1] = gW1[1];
+        } else {
+          row[(rg == NF / 2 ? OFF_B1 : OFF_B2) + u] = gb;
+        }
+        if (tid < NO * NH + NO) row[OFF_W3 + tid] = gW3;
+        if (tid >= TRAIN_THREADS - 32) {
+          float l = sl[tid % 32];
+#pragma unroll
+          for (int o = 16; o > 0; o >>= 1) l += __shfl_down_sync(0xffffffffu, l, o);
+          if (tid % 32 == 0) row[NPARAM] = l;
+        }
+        __syncthreads();
       }
+      if (!grid_sync(mine < last)) return;
+      // this CTA's sums over the tiles
+#pragma unroll
+      for (int i = 0; i < PPT; ++i) {
+        const int q = q0 + tid + TRAIN_THREADS * i;
+        if (q < q1) {
+          const float* src = a.part + q;
+          for (int t = first; t < last; t += 16, src += 16 * GSTRIDE) {
+            float v[16];
+#pragma unroll
+            for (int k = 0; k < 16; ++k) v[k] = t + k < last ? __ldcg(src + k * GSTRIDE) : 0.0f;
+#pragma unroll
+            for (int k = 0; k < 16; ++k) sum[i] += v[k];
+          }
+        }
+      }
+      if (last < ntile && !grid_sync(false)) return;  // the rows are read
+    }
+    if (TRAIN) {
+      const float2 c = a.c12[step];
+      const float inv = 1.0f / nb;
+#pragma unroll
+      for (int i = 0; i < PPT; ++i) {
+        const int q = q0 + tid + TRAIN_THREADS * i;
+        const float g = sum[i] * inv;
+        if (q < min(q1, NPARAM)) {
+          m1[i] = fmaf(a.b1, m1[i], (1.0f - a.b1) * g);
+          m2[i] = fmaf(a.b2, m2[i], (1.0f - a.b2) * g * g);
+          p[i] -= a.lr * (m1[i] / c.x) / (sqrtf(m2[i] / c.y) + 1e-8f);
+          a.params[q] = p[i];
+        } else {
+          p[i] = sum[i];
+        }
+      }
+      if (step + 1 < steps) {
+        if (!grid_sync(false)) return;
+        load_weights();
+        __syncthreads();
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < PPT; ++i) {
+        const int q = q0 + tid + TRAIN_THREADS * i;
+        if (q < min(q1, NPARAM)) a.grad[q] = sum[i];
+        p[i] = sum[i];
+      }
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < PPT; ++i) {
+    const int q = q0 + tid + TRAIN_THREADS * i;
+    if (q >= q1) continue;
+    if (q == NPARAM) {
+      *a.loss = p[i];
+    } else if (TRAIN) {
+      a.m1[q] = m1[i];
+      a.m2[q] = m2[i];
     }
   }
 }
@@ -1112,9 +1165,15 @@ extern "C" int imcom_gpu_bisect_kappa_learned(imcom_ctx* ctx, int UnotS, double 
   return copy_pixel_outputs(ctx, K_out, US_out, nevals_out);
 }
 
-// CTAs of the training kernel: a tile of each batch at least, one per SM.
-static int train_grid(imcom_ctx* ctx, int batch) {
-  return std::max(1, std::min((batch + TB - 1) / TB, sm_count(ctx)));
+constexpr long long TRAIN_SPIN = 20000000LL;  // polls of a barrier at most
+
+// Grid of the training kernel (a tile of each batch at least, one CTA per SM) and
+// its rows, a multiple of the grid.
+static int train_grid(imcom_ctx* ctx, int batch, int* rows) {
+  const int tiles = (batch + TB - 1) / TB;
+  const int G = std::max(1, std::min(tiles, sm_count(ctx)));
+  *rows = std::max(1, std::min((tiles + G - 1) / G, TRAIN_ROWS / G)) * G;
+  return G;
 }
 
 // Gradient of the summed loss over `nsamples` samples at the given parameters
@@ -1129,12 +1188,17 @@ extern "C" int imcom_gpu_mlp_gradient(imcom_ctx* ctx, int nsamples, const float*
   if (!params) return -5;
   if (!grad_out) return -6;
   cudaSetDevice(ctx->device);
-  size_t need = ((size_t)NF * nsamples + nsamples + 2 * GSTRIDE + 64) * sizeof(float);
+  int rows = 0;
+  const int G = train_grid(ctx, nsamples, &rows);
+  // tiles' rows | gradient | parameters | loss, the barrier's count and its error |
+  // features | targets
+  size_t need = (((size_t)rows + 2) * GSTRIDE + 4 + (size_t)(NF + 1) * nsamples) * sizeof(float);
   IMC_TRY(ensure_buf(ctx, (void**)&ctx->train_buf, ctx->train_bytes, need));
-  float* dgrad = (float*)ctx->train_buf;  // 16-byte aligned, as the loss after it
-  float* dloss = dgrad + GSTRIDE;
-  float* dparams = dloss + 4;
-  float* dfeat = dparams + GSTRIDE;
+  float* dpart = (float*)ctx->train_buf;
+  float* dgrad = dpart + (size_t)rows * GSTRIDE;
+  float* dparams = dgrad + GSTRIDE;
+  float* dctl = dparams + GSTRIDE;
+  float* dfeat = dctl + 4;
   float* dtarget = dfeat + (size_t)NF * nsamples;
   IMC_CUDA(cudaMemcpyAsync(dfeat, feat, (size_t)NF * nsamples * sizeof(float),
                            cudaMemcpyHostToDevice, ctx->stream));
@@ -1142,23 +1206,34 @@ extern "C" int imcom_gpu_mlp_gradient(imcom_ctx* ctx, int nsamples, const float*
                            ctx->stream));
   IMC_CUDA(cudaMemcpyAsync(dparams, params, NPARAM * sizeof(float), cudaMemcpyHostToDevice,
                            ctx->stream));
-  IMC_CUDA(cudaMemsetAsync(dgrad, 0, (GSTRIDE + 4) * sizeof(float), ctx->stream));
+  IMC_CUDA(cudaMemsetAsync(dctl, 0, 4 * sizeof(float), ctx->stream));
   TrainArgs ta{};
   ta.params = dparams;
   ta.feat = dfeat;
   ta.nall = ta.nsamples = ta.batch = nsamples;
   ta.target = dtarget;
+  ta.part = dpart;
+  ta.rows = rows;
   ta.grad = dgrad;
-  ta.loss = dloss;
-  mlp_train_kernel<false>
-      <<<train_grid(ctx, nsamples), TRAIN_THREADS, 0, ctx->stream>>>(ta);
+  ta.loss = dctl;
+  ta.arrived = (unsigned*)(dctl + 1);
+  ta.err = (int*)(dctl + 2);
+  ta.spin = TRAIN_SPIN;
+  void* args[] = {&ta};
+  IMC_CUDA(cudaLaunchCooperativeKernel((void*)mlp_train_kernel<false>, G, TRAIN_THREADS, args, 0,
+                                       ctx->stream));
   IMC_LAUNCH();
+  struct {
+    float loss;
+    int arrived, err, pad;
+  } ctl;
+  IMC_CUDA(cudaMemcpyAsync(&ctl, dctl, sizeof ctl, cudaMemcpyDeviceToHost, ctx->stream));
+  IMC_CUDA(cudaStreamSynchronize(ctx->stream));
+  if (ctl.err) return set_err(ctx, IMCOM_ERR_CUDA, "training's grid barrier timed out");
   IMC_CUDA(cudaMemcpyAsync(grad_out, dgrad, NPARAM * sizeof(float), cudaMemcpyDeviceToHost,
                            ctx->stream));
-  float l = 0.0f;
-  IMC_CUDA(cudaMemcpyAsync(&l, dloss, sizeof(float), cudaMemcpyDeviceToHost, ctx->stream));
   IMC_CUDA(cudaStreamSynchronize(ctx->stream));
-  if (loss_out) *loss_out = l;
+  if (loss_out) *loss_out = ctl.loss;
   return 0;
 }
 
@@ -1177,14 +1252,15 @@ extern "C" int imcom_gpu_mlp_train(imcom_ctx* ctx, int nsamples, const float* fe
   cudaSetDevice(ctx->device);
   batch = std::min(batch, nsamples);
   const int steps = (nsamples + batch - 1) / batch;
-  // gradients (three, in turn) | moments | parameters | per epoch the loss, the
-  // barrier's count and its error | per-step bias corrections and the epoch's order |
-  // features | targets
-  size_t need = (6 * (size_t)GSTRIDE + 4 * (size_t)epochs + 2 * (size_t)steps +
+  int rows = 0;
+  const int G = train_grid(ctx, batch, &rows);
+  // tiles' rows | moments | parameters | per epoch the loss, the barrier's count and
+  // its error | per-step bias corrections and the epoch's order | features | targets
+  size_t need = (((size_t)rows + 3) * GSTRIDE + 4 * (size_t)epochs + 2 * (size_t)steps +
                  (size_t)(NF + 2) * nsamples) * sizeof(float);
   IMC_TRY(ensure_buf(ctx, (void**)&ctx->train_buf, ctx->train_bytes, need));
-  float* dgrad = (float*)ctx->train_buf;
-  float* dm1 = dgrad + 3 * GSTRIDE;
+  float* dpart = (float*)ctx->train_buf;
+  float* dm1 = dpart + (size_t)rows * GSTRIDE;
   float* dm2 = dm1 + GSTRIDE;
   float* dparams = dm2 + GSTRIDE;
   float* dctl = dparams + GSTRIDE;
@@ -1213,8 +1289,8 @@ extern "C" int imcom_gpu_mlp_train(imcom_ctx* ctx, int nsamples, const float* fe
   };
   const float b1 = 0.9f, b2 = 0.999f;
   int step = 0;
-  TrainArgs ta{dparams, dfeat, nsamples, dtarget, didx, nsamples, batch, dgrad, nullptr, dm1, dm2,
-               dc12, lr, b1, b2, nullptr, nullptr, 20000000LL};
+  TrainArgs ta{dparams, dfeat, nsamples, dtarget, didx, nsamples, batch, dpart, rows, nullptr,
+               nullptr, dm1, dm2, dc12, lr, b1, b2, nullptr, nullptr, TRAIN_SPIN};
   for (int ep = 0; ep < epochs; ++ep) {
     for (int q = 0; q < nsamples; ++q) order[q] = q;
     for (int q = nsamples - 1; q > 0; --q) std::swap(order[q], order[rnd() % (q + 1)]);
@@ -1225,13 +1301,12 @@ extern "C" int imcom_gpu_mlp_train(imcom_ctx* ctx, int nsamples, const float* fe
     }
     IMC_CUDA(cudaMemcpyAsync(dc12, host.data(), host.size() * sizeof(int), cudaMemcpyHostToDevice,
                              ctx->stream));
-    IMC_CUDA(cudaMemsetAsync(dgrad, 0, 3 * GSTRIDE * sizeof(float), ctx->stream));
     ta.loss = dctl + 4 * (size_t)ep;
     ta.arrived = (unsigned*)(ta.loss + 1);
     ta.err = (int*)(ta.loss + 2);
     void* args[] = {&ta};
-    IMC_CUDA(cudaLaunchCooperativeKernel((void*)mlp_train_kernel<true>, train_grid(ctx, batch),
-                                         TRAIN_THREADS, args, 0, ctx->stream));
+    IMC_CUDA(cudaLaunchCooperativeKernel((void*)mlp_train_kernel<true>, G, TRAIN_THREADS, args, 0,
+                                         ctx->stream));
     IMC_LAUNCH();
   }
   std::vector<float> ctl(4 * (size_t)epochs);
