@@ -33,6 +33,7 @@
 
 #include "common.cuh"
 #include "solve.cuh"
+#include "train_ctl.h"
 #include "usum.cuh"
 
 namespace imcom {
@@ -1190,15 +1191,15 @@ extern "C" int imcom_gpu_mlp_gradient(imcom_ctx* ctx, int nsamples, const float*
   cudaSetDevice(ctx->device);
   int rows = 0;
   const int G = train_grid(ctx, nsamples, &rows);
-  // tiles' rows | gradient | parameters | loss, the barrier's count and its error |
-  // features | targets
-  size_t need = (((size_t)rows + 2) * GSTRIDE + 4 + (size_t)(NF + 1) * nsamples) * sizeof(float);
+  // tiles' rows | gradient | parameters | control words | features | targets
+  size_t need = (((size_t)rows + 2) * GSTRIDE + (size_t)(NF + 1) * nsamples) * sizeof(float) +
+                sizeof(TrainCtl);
   IMC_TRY(ensure_buf(ctx, (void**)&ctx->train_buf, ctx->train_bytes, need));
   float* dpart = (float*)ctx->train_buf;
   float* dgrad = dpart + (size_t)rows * GSTRIDE;
   float* dparams = dgrad + GSTRIDE;
-  float* dctl = dparams + GSTRIDE;
-  float* dfeat = dctl + 4;
+  TrainCtl* dctl = (TrainCtl*)(dparams + GSTRIDE);
+  float* dfeat = (float*)(dctl + 1);
   float* dtarget = dfeat + (size_t)NF * nsamples;
   IMC_CUDA(cudaMemcpyAsync(dfeat, feat, (size_t)NF * nsamples * sizeof(float),
                            cudaMemcpyHostToDevice, ctx->stream));
@@ -1206,7 +1207,7 @@ extern "C" int imcom_gpu_mlp_gradient(imcom_ctx* ctx, int nsamples, const float*
                            ctx->stream));
   IMC_CUDA(cudaMemcpyAsync(dparams, params, NPARAM * sizeof(float), cudaMemcpyHostToDevice,
                            ctx->stream));
-  IMC_CUDA(cudaMemsetAsync(dctl, 0, 4 * sizeof(float), ctx->stream));
+  IMC_CUDA(cudaMemsetAsync(dctl, 0, sizeof(TrainCtl), ctx->stream));
   TrainArgs ta{};
   ta.params = dparams;
   ta.feat = dfeat;
@@ -1215,21 +1216,18 @@ extern "C" int imcom_gpu_mlp_gradient(imcom_ctx* ctx, int nsamples, const float*
   ta.part = dpart;
   ta.rows = rows;
   ta.grad = dgrad;
-  ta.loss = dctl;
-  ta.arrived = (unsigned*)(dctl + 1);
-  ta.err = (int*)(dctl + 2);
+  ta.loss = &dctl->loss;
+  ta.arrived = &dctl->arrived;
+  ta.err = &dctl->err;
   ta.spin = TRAIN_SPIN;
   void* args[] = {&ta};
   IMC_CUDA(cudaLaunchCooperativeKernel((void*)mlp_train_kernel<false>, G, TRAIN_THREADS, args, 0,
                                        ctx->stream));
   IMC_LAUNCH();
-  struct {
-    float loss;
-    int arrived, err, pad;
-  } ctl;
+  TrainCtl ctl;
   IMC_CUDA(cudaMemcpyAsync(&ctl, dctl, sizeof ctl, cudaMemcpyDeviceToHost, ctx->stream));
   IMC_CUDA(cudaStreamSynchronize(ctx->stream));
-  if (ctl.err) return set_err(ctx, IMCOM_ERR_CUDA, "training's grid barrier timed out");
+  if (train_failed(&ctl, 1)) return set_err(ctx, IMCOM_ERR_CUDA, "training's grid barrier timed out");
   IMC_CUDA(cudaMemcpyAsync(grad_out, dgrad, NPARAM * sizeof(float), cudaMemcpyDeviceToHost,
                            ctx->stream));
   IMC_CUDA(cudaStreamSynchronize(ctx->stream));
@@ -1254,17 +1252,17 @@ extern "C" int imcom_gpu_mlp_train(imcom_ctx* ctx, int nsamples, const float* fe
   const int steps = (nsamples + batch - 1) / batch;
   int rows = 0;
   const int G = train_grid(ctx, batch, &rows);
-  // tiles' rows | moments | parameters | per epoch the loss, the barrier's count and
-  // its error | per-step bias corrections and the epoch's order | features | targets
-  size_t need = (((size_t)rows + 3) * GSTRIDE + 4 * (size_t)epochs + 2 * (size_t)steps +
-                 (size_t)(NF + 2) * nsamples) * sizeof(float);
+  // tiles' rows | moments | parameters | the epochs' control words | per-step bias
+  // corrections and the epoch's order | features | targets
+  size_t need = (((size_t)rows + 3) * GSTRIDE + 2 * (size_t)steps + (size_t)(NF + 2) * nsamples) *
+                    sizeof(float) + (size_t)epochs * sizeof(TrainCtl);
   IMC_TRY(ensure_buf(ctx, (void**)&ctx->train_buf, ctx->train_bytes, need));
   float* dpart = (float*)ctx->train_buf;
   float* dm1 = dpart + (size_t)rows * GSTRIDE;
   float* dm2 = dm1 + GSTRIDE;
   float* dparams = dm2 + GSTRIDE;
-  float* dctl = dparams + GSTRIDE;
-  float2* dc12 = (float2*)(dctl + 4 * (size_t)epochs);
+  TrainCtl* dctl = (TrainCtl*)(dparams + GSTRIDE);
+  float2* dc12 = (float2*)(dctl + epochs);
   int* didx = (int*)(dc12 + steps);
   float* dfeat = (float*)(didx + nsamples);
   float* dtarget = dfeat + (size_t)NF * nsamples;
@@ -1275,7 +1273,7 @@ extern "C" int imcom_gpu_mlp_train(imcom_ctx* ctx, int nsamples, const float* fe
   IMC_CUDA(cudaMemcpyAsync(dparams, params, NPARAM * sizeof(float), cudaMemcpyHostToDevice,
                            ctx->stream));
   IMC_CUDA(cudaMemsetAsync(dm1, 0, 2 * GSTRIDE * sizeof(float), ctx->stream));
-  IMC_CUDA(cudaMemsetAsync(dctl, 0, 4 * (size_t)epochs * sizeof(float), ctx->stream));
+  IMC_CUDA(cudaMemsetAsync(dctl, 0, epochs * sizeof(TrainCtl), ctx->stream));
   // shuffled order per epoch (host xorshift, reproducible from the seed)
   std::vector<int> host(2 * (size_t)steps + nsamples);
   float* c12 = (float*)host.data();
@@ -1301,24 +1299,25 @@ extern "C" int imcom_gpu_mlp_train(imcom_ctx* ctx, int nsamples, const float* fe
     }
     IMC_CUDA(cudaMemcpyAsync(dc12, host.data(), host.size() * sizeof(int), cudaMemcpyHostToDevice,
                              ctx->stream));
-    ta.loss = dctl + 4 * (size_t)ep;
-    ta.arrived = (unsigned*)(ta.loss + 1);
-    ta.err = (int*)(ta.loss + 2);
+    ta.loss = &dctl[ep].loss;
+    ta.arrived = &dctl[ep].arrived;
+    ta.err = &dctl[ep].err;
     void* args[] = {&ta};
     IMC_CUDA(cudaLaunchCooperativeKernel((void*)mlp_train_kernel<true>, G, TRAIN_THREADS, args, 0,
                                          ctx->stream));
     IMC_LAUNCH();
   }
-  std::vector<float> ctl(4 * (size_t)epochs);
-  IMC_CUDA(cudaMemcpyAsync(ctl.data(), dctl, ctl.size() * sizeof(float), cudaMemcpyDeviceToHost,
+  std::vector<TrainCtl> ctl(epochs);
+  IMC_CUDA(cudaMemcpyAsync(ctl.data(), dctl, ctl.size() * sizeof(TrainCtl), cudaMemcpyDeviceToHost,
                            ctx->stream));
+  IMC_CUDA(cudaStreamSynchronize(ctx->stream));
+  // the caller's parameters stay as they are
+  if (train_failed(ctl.data(), epochs))
+    return set_err(ctx, IMCOM_ERR_CUDA, "training's grid barrier timed out");
   IMC_CUDA(cudaMemcpyAsync(params, dparams, NPARAM * sizeof(float), cudaMemcpyDeviceToHost,
                            ctx->stream));
   IMC_CUDA(cudaStreamSynchronize(ctx->stream));
-  for (int ep = 0; ep < epochs; ++ep)
-    if (ctl[4 * (size_t)ep + 2] != 0.0f)
-      return set_err(ctx, IMCOM_ERR_CUDA, "training's grid barrier timed out");
   if (loss_out)
-    for (int ep = 0; ep < epochs; ++ep) loss_out[ep] = ctl[4 * (size_t)ep] / nsamples;
+    for (int ep = 0; ep < epochs; ++ep) loss_out[ep] = ctl[ep].loss / nsamples;
   return 0;
 }
