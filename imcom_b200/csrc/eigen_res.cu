@@ -20,6 +20,9 @@
 // reader polls the data itself, with no fence, flag or barrier.  Two buffers
 // by column parity suffice: a CTA publishes column j+2 only after it has read
 // every value of column j+1, which each owner wrote after reading column j.
+// A CTA whose last row is j+1 owns none of them, so it publishes column j and
+// returns without reading it; column j of V, d, e and tau is written by the
+// owner of row j+2 (res_rows.h).
 // Polls are bounded: a value that does not come sets the error word.
 //
 // What bounds it: the latency of one exchange (about 1500 cycles for 600
@@ -34,6 +37,7 @@
 
 #include "common.cuh"
 #include "eigen.cuh"
+#include "res_rows.h"
 #include "tagged.cuh"
 
 namespace imcom {
@@ -43,12 +47,6 @@ namespace {
 
 constexpr int RT = 256;      // threads per CTA
 constexpr int RW = RT / 32;  // warps
-// Rows go to the CTAs in pairs: a pair's records are 64 consecutive bytes,
-// written by one store instruction.  (Measured on an exchange alone, 148 CTAs
-// publishing 1776 16-byte values: 8000 cycles when every value is its own
-// store into a line shared with 7 other CTAs, 2190 with 64 bytes per store,
-// 2100 with whole 128-byte lines.)
-constexpr int RBLK = 2;
 
 struct ResArgs {
   const double* A;  // lower triangle valid for rows and columns k0 .. n-1
@@ -158,11 +156,9 @@ __global__ void __launch_bounds__(RT, 1) trd_resident_kernel(ResArgs a) {
   const int q = blockIdx.x, G = gridDim.x;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const int S = a.n - a.k0, ldS = (S + 63) & ~63, k0 = a.k0;
-  // own rows i = 0 .. nrow-1, ascending: row(i) = 4 (q + G (i / 4)) + i % 4;
-  // the rows past S of the last block are zero
-  auto row = [&](int i) { return RBLK * (q + G * (i / RBLK)) + i % RBLK; };
-  int nrow = a.nrow;
-  while (nrow > 0 && row(nrow - 1) >= S) --nrow;
+  // own rows; those past S of the last block are zero
+  const ResRows rows(q, G, S, a.nrow);
+  const int nrow = rows.nrow;
   const int nblk = (nrow + RBLK - 1) / RBLK;
   extern __shared__ __align__(16) double rsm[];
   double* As = rsm;                                     // [nrow][ldS], columns at res_pos, zero past S
@@ -178,7 +174,7 @@ __global__ void __launch_bounds__(RT, 1) trd_resident_kernel(ResArgs a) {
   // across the columns left of it
   const double* A0 = a.A + (long long)k0 * (a.lda + 1);
   for (int i = 0; i < RBLK * nblk; ++i) {
-    const int r = row(i);
+    const int r = rows.row(i);
     for (int c = tid; c < ldS; c += RT) {
       double v = 0.0;
       if (c < S && r < S)
@@ -208,15 +204,14 @@ __global__ void __launch_bounds__(RT, 1) trd_resident_kernel(ResArgs a) {
 
   // of the pending column: w_r = c1 z_r + c2 A(r, j+1) + c3 x_r, v_r = scl x_r
   double c1 = 0.0, c2 = 0.0, c3 = 0.0, scl = 0.0, w1 = 0.0;
-  int i0 = 0, r0 = row(0);  // first own row below row j
+  int i0 = 0, r0 = rows.row(0);  // first own row below row j
   for (int j = 0; j < S - 1; ++j) {
     const unsigned tag = (unsigned)(j + 1);
     if (r0 <= j) {
+      r0 = rows.after(i0, r0);
       ++i0;
-      r0 += (i0 % RBLK) ? 1 : 1 + RBLK * (G - 1);
     }
-    if (i0 >= nrow) return;  // every own row is done; nothing left to publish
-    const bool pub = r0 == j + 1;
+    const bool pub = rows.writes(j, i0, r0);
     const int kmin = (j + 1) / (2 * RT);  // the slots before it are left of column j+1
     const int p1 = res_pos(j + 1);
     const bool at1 = tid + RT * kmin == p1 >> 1;  // holds column j+1, in slot kmin
@@ -257,13 +252,14 @@ __global__ void __launch_bounds__(RT, 1) trd_resident_kernel(ResArgs a) {
     for (int t = 2 * i0 + tid; t < 2 * nrow; t += RT) {
       const int i = t >> 1;
       const double rv = As[(size_t)i * ldS + p1], zv = sum_warps(red + i * RW);
-      st_tagged(rec + 2 * row(i) + (t & 1), (t & 1) ? rv : zv, tag);
+      st_tagged(rec + 2 * rows.row(i) + (t & 1), (t & 1) ? rv : zv, tag);
       if (!(t & 1)) {
         const double4 o = xzr[i];  // of column j-1
         const double vr = scl * o.x, wr = fma(c1, o.y, fma(c2, o.z, c3 * o.x));
         xzr[i] = make_double4(j ? fma(-w1, vr, o.z - wr) : o.x, zv, rv, 0.0);
       }
     }
+    if (rows.retires(j, i0, r0)) return;
     if (wid == RW - 1) {
       // Householder reflector of x (LAPACK dlarfg), while the records travel
       const double xn2 = sum_warps(redn);
