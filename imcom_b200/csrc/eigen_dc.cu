@@ -265,6 +265,19 @@ struct Node {
   int s, n1, nm;  // first row, left child size, node size
 };
 
+// dt = d, and bit 16 of *err where d or e is not finite (a matrix that is not, or
+// whose reduction overflowed): nothing below runs on such values.
+__global__ void __launch_bounds__(1024) dc_input_kernel(const double* d, const double* e, int n,
+                                                        double* dt, int* err) {
+  bool bad = false;
+  for (int i = threadIdx.x; i < n; i += 1024) {
+    const double v = d[i];
+    bad |= !isfinite(v) || (i < n - 1 && !isfinite(e[i]));
+    dt[i] = v;
+  }
+  if (__syncthreads_or(bad) && threadIdx.x == 0) atomicOr(err, 16);
+}
+
 // Tearing: d(s-1) -= |e(s-1)|, d(s) -= |e(s-1)| at every split point (a thread
 // each: leaves hold LEAF / 2 rows or more, so no two splits share one).
 __global__ void tear_kernel(double* dt, const double* e, const int* splits, int nsplit) {
@@ -398,6 +411,7 @@ __global__ void __launch_bounds__(256) leaf_jacobi_kernel(const Node* nodes, con
     if (sweep == max_sweeps - 1 && tid == 0) atomicOr(err, 2);
   }
   // ascending order: the rank of each value (ties by index)
+  if (tid < m) s_idx[tid] = tid;
   __syncthreads();
   if (tid < m) {
     const double v = Am[tid][tid];
@@ -1149,7 +1163,7 @@ static int sytrd_launches(imcom_ctx* ctx, DMat& Aw, DMat& Vall, double* d, doubl
 // replayed as a CUDA graph once the same size and buffers come back: the
 // first call at a key runs it directly, the second captures and instantiates
 // it, later calls launch the graph.  A capture the driver refuses leaves the
-// direct path in place.
+// direct path in place.  A timed-out exchange leaves its word set; the caller reads it.
 static int sytrd_gpu(imcom_ctx* ctx, DMat& Aw, DMat& Vall, double* d, double* e, double* tau,
                      double* W, long long ldw, int* err, void* panbuf, long long spin, double* XY,
                      int res_max, void* resbuf) {
@@ -1212,11 +1226,6 @@ static int sytrd_gpu(imcom_ctx* ctx, DMat& Aw, DMat& Vall, double* d, double* e,
     IMC_TRY(sytrd_launches(ctx, Aw, Vall, d, e, tau, W, ldw, err, panbuf, spin, XY,
                            tail_ctas, tail_max, res_max, resbuf, false));
   }
-  // a timed-out exchange ends the factorisation with an error
-  int h = 0;
-  IMC_CUDA(cudaMemcpyAsync(&h, err, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
-  IMC_CUDA(cudaStreamSynchronize(ctx->stream));
-  if (h) return set_err(ctx, IMCOM_ERR_EIGEN, "tridiagonalisation grid barrier timed out");
   return 0;
 }
 
@@ -1265,7 +1274,7 @@ int eigen_dc(imcom_ctx* ctx, const DMat& A, DMat& Wout, double* wout) {
   const size_t npair_bt = (nblk_bt + 1) / 2;
   size_t o_T = take(npair_bt * 4 * NBB * NBB * 8), o_G = take(npair_bt * 4 * NBB * NBB * 8);
   size_t o_X = take((size_t)2 * NBB * ld * 8 * 2);
-  size_t o_err = take(64), o_terr = take(64);
+  size_t o_err = take(64);
   size_t o_2s = take(two ? twostage_bytes(n) : 0);
   IMC_TRY(eig_buf(ctx, off + 256));
   char* base = (char*)ew->buf;
@@ -1279,7 +1288,8 @@ int eigen_dc(imcom_ctx* ctx, const DMat& A, DMat& Wout, double* wout) {
   double* Tb = (double*)(base + o_T);
   double* Gb = (double*)(base + o_G);
   double* Xb = (double*)(base + o_X);
-  int* derr = (int*)(base + o_err);
+  int* derr = (int*)(base + o_err);  // the divide and conquer's, and the exchanges'
+  int* terr = derr + 1;
   IMC_CUDA(cudaMemsetAsync(derr, 0, 64, ctx->stream));
 
   // ---- 1. tridiagonalisation ----
@@ -1294,9 +1304,19 @@ int eigen_dc(imcom_ctx* ctx, const DMat& A, DMat& Wout, double* wout) {
     IMC_TRY(twostage_tridiag(ctx, Aw, Vall, d, e, tau, Wp, ldw, (double*)(base + o_XY),
                              base + o_2s, spin));
   else
-    IMC_TRY(sytrd_gpu(ctx, Aw, Vall, d, e, tau, Wp, ldw, (int*)(base + o_terr),
+    IMC_TRY(sytrd_gpu(ctx, Aw, Vall, d, e, tau, Wp, ldw, terr,
                       panels ? base + o_pan : nullptr, spin, (double*)(base + o_XY), res_max,
                       base + o_res));
+  dc_input_kernel<<<1, 1024, 0, ctx->stream>>>(d, e, n, dt, derr);
+  IMC_LAUNCH();
+  {
+    int h[2] = {};
+    IMC_CUDA(cudaMemcpyAsync(h, derr, sizeof h, cudaMemcpyDeviceToHost, ctx->stream));
+    IMC_CUDA(cudaStreamSynchronize(ctx->stream));
+    if (h[1]) return set_err(ctx, IMCOM_ERR_EIGEN, "tridiagonalisation grid barrier timed out");
+    if (h[0])
+      return set_err(ctx, IMCOM_ERR_EIGEN, "the tridiagonal matrix has a non-finite entry");
+  }
   stage_end(ctx, ST_EIG_TRD);
   stage_begin(ctx, ST_EIG_DC);
 
@@ -1319,7 +1339,6 @@ int eigen_dc(imcom_ctx* ctx, const DMat& A, DMat& Wout, double* wout) {
   std::vector<int> splits;
   for (size_t L = 0; L + 1 < levels.size(); ++L)
     for (const Node& x : levels[L]) splits.push_back(x.s + x.n1);
-  IMC_CUDA(cudaMemcpyAsync(dt, d, n * 8, cudaMemcpyDeviceToDevice, ctx->stream));
   if (!splits.empty()) {
     IMC_CUDA(cudaMemcpyAsync(dsplit, splits.data(), splits.size() * 4, cudaMemcpyHostToDevice,
                              ctx->stream));

@@ -1,0 +1,61 @@
+"""Matrices at the ends of the range in the eigensolver (csrc/eigen_dc.cu): entries
+that are not finite, or whose reduction overflows, end the call with an error on every
+path of the tridiagonalisation, and the context solves the next matrix.
+
+Tolerance: a backward-stable method gives eigenvalues, residual and orthogonality
+within c n eps |A|_2; c = 10, the threshold of LAPACK's own test ratios."""
+import numpy as np
+import pytest
+
+from imcom_b200 import EIGH_TWOSTAGE, ImcomError, Solver
+from imcom_b200.api import OPT_SM_SHARE, OPT_TAIL_CTAS
+
+pytestmark = pytest.mark.gpu
+
+EPS = 2.0 ** -53
+IMCOM_ERR_EIGEN = 5
+
+
+def _set(s, n):
+    x = np.arange(n, dtype=float)
+    s.set_inputs(x, x, np.ones(n, dtype=np.int32), x[:1], x[:1], None, None, 1.0, 1.0)
+
+
+def _check(s, A):
+    n = A.shape[0]
+    s.load_A(np.asfortranarray(A))
+    Q, L, _ = s.eigen_A()
+    bound = 10 * n * EPS * np.linalg.norm(A, 2)
+    assert np.abs(L - np.linalg.eigvalsh(A)[::-1]).max() <= bound
+    assert np.linalg.norm(A @ Q - Q * L, 2) <= bound
+    assert np.linalg.norm(Q.T @ Q - np.eye(n), 2) <= 10 * n * EPS
+
+
+def _matrix(n):
+    rng = np.random.default_rng(n)
+    V = rng.standard_normal((n, n))
+    return V @ V.T
+
+
+@pytest.mark.parametrize("n,tail,share,two", [(2, 0, 0, False), (20, 0, 0, False), (70, 0, 0, False),
+                                              (300, 8, 0, False), (300, 16, 0, False),
+                                              (300, -1, 0, False), (300, 0, 3, False),
+                                              (300, 0, 24, False), (2100, 0, 0, False),
+                                              (300, 0, 0, True)])
+@pytest.mark.parametrize("bad", [np.nan, np.inf, 1e200])
+def test_not_finite_is_an_error(n, tail, share, two, bad):
+    A = _matrix(n)
+    with Solver(0) as s:
+        if two:
+            s.set_eigensolver(EIGH_TWOSTAGE)
+        s.set_option(OPT_TAIL_CTAS, tail)
+        s.set_option(OPT_SM_SHARE, share)
+        _set(s, n)
+        B = A * bad if bad == 1e200 and n > 2 else A.copy()
+        if bad != 1e200 or n == 2:
+            B[n // 2, n // 3] = B[n // 3, n // 2] = np.nan if n == 2 else bad
+        s.load_A(np.asfortranarray(B))
+        with pytest.raises(ImcomError) as ei:
+            s.eigen_A()
+        assert ei.value.status == IMCOM_ERR_EIGEN
+        _check(s, A)
