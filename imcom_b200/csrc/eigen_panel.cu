@@ -342,7 +342,8 @@ __global__ void __launch_bounds__(PT, 1) trd_panel_kernel(PanelArgs a) {
       if (!owner) continue;
       // x^T A22 x and (A22 x)(j+1); then alpha2 = -1/2 tau^2 v^T y and w(j+1), with
       // v^T y = v^T y0 - 2 (V^T v).(W^T v) and v^T y0 = scl^2 x^T A22 x + 2 scl delta
-      // (A22 x)(j+1) + delta^2 A(j+1, j+1)
+      // (A22 x)(j+1) + delta^2 A(j+1, j+1) (scl is not squared: that overflows for a
+      // column of norm 1e-155 and less)
       double xax = 0.0, y1 = 0.0;
       const int nrun = cur.cta(cur.end(0) - cur.ch0 - 1) + 1, tot = nrun + cur.RB;
       for (int m = lane; m < max(G, tot); m += 160) {
@@ -363,7 +364,7 @@ __global__ void __launch_bounds__(PT, 1) trd_panel_kernel(PanelArgs a) {
       xax = wsum(xax);
       y1 = wsum(y1);
       const double y1v = sc_scl * y1 + sc_delta * a11;
-      const double vty = sc_scl * sc_scl * xax + 2.0 * sc_scl * sc_delta * y1 + sc_delta * sc_delta * a11;
+      const double vty = sc_scl * (sc_scl * xax + 2.0 * sc_delta * y1) + sc_delta * sc_delta * a11;
       const double al2 = -0.5 * sc_t * sc_t * (vty - 2.0 * qp);
       if (lane == 0) {
         s_al2 = al2;

@@ -357,11 +357,12 @@ __global__ void __launch_bounds__(RT, 1) trd_resident_kernel(ResArgs a) {
     if (lane == 0) red2[wid] = xz;
     __syncthreads();
     if (s_fail) return;
-    // v^T y = scl^2 x^T A x + 2 scl delta (A x)(j+1) + delta^2 A(j+1, j+1)
+    // v^T y = scl^2 x^T A x + 2 scl delta (A x)(j+1) + delta^2 A(j+1, j+1); scl is not
+    // squared: that overflows for a column of norm 1e-155 and less
     const double t = s_sc.t, delta = s_sc.delta, z1 = s_z1, r1 = s_r1;
     scl = s_sc.scl;
     xz = sum_warps(red2);
-    const double vty = fma(scl * scl, xz, delta * fma(2.0 * scl, z1, delta * r1));
+    const double vty = fma(scl, fma(scl, xz, 2.0 * delta * z1), delta * (delta * r1));
     const double a2 = -0.5 * t * t * vty;
     c1 = t * scl;
     c2 = t * delta;

@@ -59,3 +59,30 @@ def test_not_finite_is_an_error(n, tail, share, two, bad):
             s.eigen_A()
         assert ei.value.status == IMCOM_ERR_EIGEN
         _check(s, A)
+
+
+# A column whose squares are subnormal: its squared norm (and x^T A x against |A|) is a
+# sum of n numbers, each rounded by up to 2^-1075, so the reflector and the update are
+# exact to n 2^-1075 / |x|^2; 16 of these for the reflector's two sides, the update's
+# terms and the two sums.
+@pytest.mark.parametrize("n,split,tail", [(40, 1, 0), (40, 20, 0), (300, 1, 0), (300, 45, 0),
+                                          (300, 1, -1), (300, 45, -1), (300, 45, 16),
+                                          (2100, 1, 0), (2100, 40, 0)])
+@pytest.mark.parametrize("tiny", [1e-153, 1e-155, 1e-156, 1e-157, 1e-158])
+def test_tiny_columns(n, split, tail, tiny):
+    rng = np.random.default_rng(n + split)
+    A = _matrix(n) / n
+    A[:split, split:] = tiny * rng.uniform(1, 2, (split, n - split))
+    A[split:, :split] = A[:split, split:].T
+    # |x|^2 of the first block's last column: its couplings through an orthogonal map
+    norm2 = np.linalg.svd(A[:split, split:] / tiny, compute_uv=False).min() ** 2
+    rel = 10 * n * EPS + 16 * n * (2.0 ** -1000 / tiny / tiny * 2.0 ** -75) / norm2
+    with Solver(0) as s:
+        s.set_option(OPT_TAIL_CTAS, tail)
+        _set(s, n)
+        s.load_A(np.asfortranarray(A))
+        Q, L, _ = s.eigen_A()
+    norm = np.linalg.norm(A, 2)
+    assert np.abs(L - np.linalg.eigvalsh(A)[::-1]).max() <= rel * norm
+    assert np.linalg.norm(A @ Q - Q * L, 2) <= rel * norm
+    assert np.linalg.norm(Q.T @ Q - np.eye(n), 2) <= rel
