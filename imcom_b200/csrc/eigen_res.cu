@@ -408,21 +408,24 @@ size_t res_smem(int S, int G) {
 
 size_t res_rec_bytes(int S) { return 4 * (size_t)((S + 63) & ~63) * sizeof(ulonglong2); }
 
+size_t res_limit(int dev) {
+  int optin = 0;
+  cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  return optin > 2048 ? (size_t)optin - 1024 : 0;  // room for static shared
+}
+
 template <int KP>
 int launch_res(imcom_ctx* ctx, ResArgs& a, int G, size_t smem) {
+  // the limit, not this order's need: the attribute is process-wide, and contexts on
+  // other threads must not lower it under one another's launches
   IMC_CUDA(cudaFuncSetAttribute(trd_resident_kernel<KP>,
-                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+                                cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)res_limit(ctx->device)));
   void* args[] = {&a};
   IMC_CUDA(cudaLaunchCooperativeKernel((void*)trd_resident_kernel<KP>, G, RT, args, smem,
                                        ctx->stream));
   IMC_LAUNCH();
   return 0;
-}
-
-size_t res_limit(int dev) {
-  int optin = 0;
-  cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-  return optin > 2048 ? (size_t)optin - 1024 : 0;  // room for static shared
 }
 
 }  // namespace
