@@ -258,6 +258,72 @@ __global__ void set_last_diag_kernel(const double* A, long long lda, int n, doub
   d[n - 1] = A[(n - 1) + (long long)(n - 1) * lda];
 }
 
+// Magnitudes within 2^+-RANGE are left alone: products of three (x^T A x) and squares
+// of their ratios to a gap or to z (EPS of them at least) stay in range.
+constexpr int RANGE = 100;
+
+// The power of two to multiply values of the order of `mag` by.
+__device__ __forceinline__ int range_shift(double mag) {
+  if (!(mag > 0.0) || !isfinite(mag)) return 0;
+  const int E = ilogb(mag);
+  return E < -RANGE || E > RANGE ? -max(-1000, min(1000, E)) : 0;
+}
+
+// The working copy of A, and the bits of the largest magnitude in its lower triangle
+// (zero before).
+__global__ void __launch_bounds__(256) copy_max_kernel(const double* __restrict__ A, long long lda,
+                                                       double* __restrict__ B, long long ldb,
+                                                       int n, unsigned long long* big) {
+  __shared__ double s_max[8];
+  double m = 0.0;
+  for (int c = blockIdx.x; c < n; c += gridDim.x) {
+    const double* a = A + (long long)c * lda;
+    double* b = B + (long long)c * ldb;
+    for (int r = 2 * threadIdx.x; r < n; r += 512) {
+      if (r + 1 < n) {
+        const double2 v = *(const double2*)(a + r);
+        *(double2*)(b + r) = v;
+        if (r >= c) m = fmax(m, fabs(v.x));
+        if (r + 1 >= c) m = fmax(m, fabs(v.y));
+      } else {
+        const double v = a[r];
+        b[r] = v;
+        m = fmax(m, fabs(v));
+      }
+    }
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
+  if ((threadIdx.x & 31) == 0) s_max[threadIdx.x >> 5] = m;
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+#pragma unroll
+  for (int w = 1; w < 8; ++w) m = fmax(m, s_max[w]);
+  atomicMax(big, (unsigned long long)__double_as_longlong(m));
+}
+
+// Rows n .. n8 - 1 of the working copy are zero (the panels read them).  Where its
+// largest entry is beyond 2^+-RANGE the copy is multiplied by 2^*shift (LAPACK dsyevd
+// scales by the norm): reflectors and updates take products of three entries.
+__global__ void __launch_bounds__(256) scale_pad_kernel(double* __restrict__ B, long long ldb, int n,
+                                                        int n8, const unsigned long long* big,
+                                                        int* shift) {
+  const int k = range_shift(__longlong_as_double((long long)*big));
+  for (int c = blockIdx.x; c < n; c += gridDim.x) {
+    double* b = B + (long long)c * ldb;
+    if (n + (int)threadIdx.x < n8) b[n + threadIdx.x] = 0.0;
+    if (k != 0)
+      for (int r = threadIdx.x; r < n; r += 256) b[r] = scalbn(b[r], k);
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) *shift = k;
+}
+
+// The eigenvalues of the matrix as it was.
+__global__ void unscale_kernel(double* w, int n, int shift) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) w[i] = scalbn(w[i], -shift);
+}
+
 // ---------------------------------------------------------------------------
 // 2. Divide and conquer
 // ---------------------------------------------------------------------------
@@ -1288,16 +1354,20 @@ int eigen_dc(imcom_ctx* ctx, const DMat& A, DMat& Wout, double* wout) {
   double* Tb = (double*)(base + o_T);
   double* Gb = (double*)(base + o_G);
   double* Xb = (double*)(base + o_X);
-  int* derr = (int*)(base + o_err);  // the divide and conquer's, and the exchanges'
+  int* derr = (int*)(base + o_err);  // the divide and conquer's, the exchanges', A's scaling
   int* terr = derr + 1;
   IMC_CUDA(cudaMemsetAsync(derr, 0, 64, ctx->stream));
 
   // ---- 1. tridiagonalisation ----
   stage_begin(ctx, ST_EIG_TRD);
-  IMC_TRY(copy_mat(ctx, A.p, A.ld, Aw.p, Aw.ld, n, n));
-  if (n % 8)  // the panels read rows up to the next multiple of 8
-    IMC_CUDA(cudaMemset2DAsync(Aw.p + n, Aw.ld * sizeof(double), 0, (8 - n % 8) * sizeof(double), n,
-                               ctx->stream));
+  {
+    unsigned long long* big = (unsigned long long*)(derr + 4);
+    const unsigned grid = (unsigned)std::min(n, 8 * sm_count(ctx));
+    copy_max_kernel<<<grid, 256, 0, ctx->stream>>>(A.p, A.ld, Aw.p, Aw.ld, n, big);
+    IMC_LAUNCH();
+    scale_pad_kernel<<<grid, 256, 0, ctx->stream>>>(Aw.p, Aw.ld, n, (n + 7) & ~7, big, derr + 2);
+    IMC_LAUNCH();
+  }
   IMC_CUDA(cudaMemsetAsync(Vall.p, 0, Vall.bytes(), ctx->stream));
   IMC_CUDA(cudaMemsetAsync(Wp, 0, (size_t)ldw * NB * 8, ctx->stream));
   if (two)
@@ -1309,13 +1379,15 @@ int eigen_dc(imcom_ctx* ctx, const DMat& A, DMat& Wout, double* wout) {
                       base + o_res));
   dc_input_kernel<<<1, 1024, 0, ctx->stream>>>(d, e, n, dt, derr);
   IMC_LAUNCH();
+  int shift = 0;
   {
-    int h[2] = {};
+    int h[3] = {};
     IMC_CUDA(cudaMemcpyAsync(h, derr, sizeof h, cudaMemcpyDeviceToHost, ctx->stream));
     IMC_CUDA(cudaStreamSynchronize(ctx->stream));
     if (h[1]) return set_err(ctx, IMCOM_ERR_EIGEN, "tridiagonalisation grid barrier timed out");
     if (h[0])
       return set_err(ctx, IMCOM_ERR_EIGEN, "the tridiagonal matrix has a non-finite entry");
+    shift = h[2];
   }
   stage_end(ctx, ST_EIG_TRD);
   stage_begin(ctx, ST_EIG_DC);
@@ -1462,6 +1534,10 @@ int eigen_dc(imcom_ctx* ctx, const DMat& A, DMat& Wout, double* wout) {
     IMC_CUDA(cudaMemcpyAsync(&h, derr, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
     IMC_CUDA(cudaStreamSynchronize(ctx->stream));
     if (h) return set_err(ctx, IMCOM_ERR_EIGEN, "divide and conquer did not converge (flags %d)", h);
+  }
+  if (shift) {
+    unscale_kernel<<<(n + 255) / 256, 256, 0, ctx->stream>>>(w, n, shift);
+    IMC_LAUNCH();
   }
 
   stage_end(ctx, ST_EIG_DC);
