@@ -505,7 +505,7 @@ struct DcWork {
   double2* rcs;
   // per node
   int *kcnt, *ndef, *nrot;
-  double* rho;
+  double *rho, *back;
 };
 
 // z, merge ranks of the two sorted child lists, scatter into sorted order.
@@ -551,6 +551,9 @@ __global__ void dc_prep_kernel(const Node* nodes, const double* w, const double*
 // (d, z) pairs, carrying the previous non-deflated entry (possibly rotated)
 // in registers.  The other warps stage the input into shared memory one
 // chunk ahead, so the walk never waits on a global-memory round trip.
+// dl and rho leave multiplied by a power of two (1 / back) where the node's values are
+// beyond 2^+-RANGE: the roots and vectors take squares of 1 / gap (a half of the matrix
+// at 1e-160 of the rest gave vectors of zeros).  The roots go back by `back`.
 constexpr int DEF_CH = 1024;
 
 __global__ void __launch_bounds__(256) dc_deflate_kernel(const Node* nodes, DcWork wk) {
@@ -580,7 +583,14 @@ __global__ void __launch_bounds__(256) dc_deflate_kernel(const Node* nodes, DcWo
     }
     __syncthreads();
   }
-  const double tol = 8.0 * EPS * fmax(sh_d[0], rho * sh_z[0]);
+  // (at least the smallest normal, which is nothing to a matrix of 2^-RANGE and more)
+  const double tol = fmax(8.0 * EPS * fmax(sh_d[0], rho * sh_z[0]), 2.2250738585072014e-308);
+  const int shift = range_shift(fmax(sh_d[0], rho));
+  const double scale = scalbn(1.0, shift);
+  if (threadIdx.x == 0) {  // every thread has read its rho
+    wk.rho[blockIdx.x] = rho * scale;
+    wk.back[blockIdx.x] = scalbn(1.0, -shift);
+  }
   // Fast path: when the cheap test below keeps every non-deflated pair (no
   // pair needs the exact rotation test), the scan keeps the non-deflated and
   // the z-deflated entries each in their order, so the output positions are
@@ -636,7 +646,7 @@ __global__ void __launch_bounds__(256) dc_deflate_kernel(const Node* nodes, DcWo
           wk.defcol[s + zo] = pm[q];
           ++zo;
         } else {
-          wk.dl[s + ko] = ds[q];
+          wk.dl[s + ko] = ds[q] * scale;
           wk.zz[s + ko] = zj;
           wk.ndcol[s + ko] = pm[q];
           ++ko;
@@ -713,7 +723,7 @@ __global__ void __launch_bounds__(256) dc_deflate_kernel(const Node* nodes, DcWo
           zp = tau;
           pp = pj;
         } else {
-          wk.dl[s + k] = dp;
+          wk.dl[s + k] = dp * scale;
           wk.zz[s + k] = zp;
           wk.ndcol[s + k] = pp;
           ++k;
@@ -727,7 +737,7 @@ __global__ void __launch_bounds__(256) dc_deflate_kernel(const Node* nodes, DcWo
   }
   if (threadIdx.x != 0) return;
   if (have) {
-    wk.dl[s + k] = dp;
+    wk.dl[s + k] = dp * scale;
     wk.zz[s + k] = zp;
     wk.ndcol[s + k] = pp;
     ++k;
@@ -837,11 +847,14 @@ __global__ void dc_secular_kernel(const Node* nodes, DcWork wk, int maxit, int* 
     }
     tau = tn;
   }
+  // the next merge ranks its values: one that is not finite ends the call
+  const bool bad = !isfinite(tau);
+  if (bad) tau = 0.0;
   if (lane == 0) {
     wk.org[s + j] = org;
     wk.tau[s + j] = tau;
-    wk.lam[s + j] = dorg + tau;
-    if (it >= maxit) atomicOr(err, 4);
+    wk.lam[s + j] = (dorg + tau) * wk.back[b];
+    if (it >= maxit || bad) atomicOr(err, 4);
   }
 }
 
@@ -1334,7 +1347,7 @@ int eigen_dc(imcom_ctx* ctx, const DMat& A, DMat& Wout, double* wout) {
   size_t o_res = take(resident_bytes(n));
   size_t o_pan = take(panels ? panel_bytes(n, panel_grid(ctx, n)) : 0);
   size_t o_split = take((size_t)n * 4), o_nodes = take((size_t)n * sizeof(Node));
-  size_t o_wk = take(((size_t)n * 8 + 16) * 9 + ((size_t)n * 4 + 16) * 8 + ((size_t)n * 24 + 32) +
+  size_t o_wk = take(((size_t)n * 8 + 16) * 10 + ((size_t)n * 4 + 16) * 8 + ((size_t)n * 24 + 32) +
                      4096);
   const size_t nblk_bt = (size_t)(n - 1 + NBB - 1) / NBB + 1;
   const size_t npair_bt = (nblk_bt + 1) / 2;
@@ -1438,6 +1451,7 @@ int eigen_dc(imcom_ctx* ctx, const DMat& A, DMat& Wout, double* wout) {
     wk.rcol = (int2*)p; adv((size_t)n * 8);
     wk.kcnt = iv(); wk.ndef = iv(); wk.nrot = iv();
     wk.rho = dv();
+    wk.back = dv();
   }
   double* w = wout;
   // leaves

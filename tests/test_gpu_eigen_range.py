@@ -118,3 +118,31 @@ def test_powers_of_two_change_nothing():
     for Q, L in out[1:]:
         assert np.array_equal(Q, out[0][0])
         assert np.array_equal(L, out[0][1])
+
+
+def _tridiagonal(n, mag):
+    rng = np.random.default_rng(n)
+    d, e = rng.uniform(1, 2, n) * mag, rng.uniform(1, 2, n - 1) * np.minimum(mag[1:], mag[:-1])
+    return np.diag(d) + np.diag(e, 1) + np.diag(e, -1)
+
+
+# Merges whose values are all far below the rest of the matrix (or far from 1 with all of
+# it): no squares of 1 / gap that leave the range.  The matrices are tridiagonal, so the
+# reduction leaves them as they are.
+@pytest.mark.parametrize("n", [20, 33, 70, 71, 140, 300])
+@pytest.mark.parametrize("tiny", [1e-80, 1e-100, 1e-160, 1e-300, 1e-310, 0.0])
+@pytest.mark.parametrize("half", ["first", "second", "middle"])
+def test_merges_of_tiny_values(n, tiny, half):
+    i = np.arange(n)
+    small = {"first": i < n // 2, "second": i >= n // 2, "middle": abs(i - n // 2) < n // 3}[half]
+    with Solver(0) as s:
+        _set(s, n)
+        _check(s, _tridiagonal(n, np.where(small, tiny, 1.0)))
+
+
+@pytest.mark.parametrize("n", [2, 20, 70, 300])
+@pytest.mark.parametrize("scale", [1e-280, 1e-120, 1e120, 1e300])
+def test_scaled_tridiagonal(n, scale):
+    with Solver(0) as s:
+        _set(s, n)
+        _check(s, _tridiagonal(n, np.full(n, scale)))
