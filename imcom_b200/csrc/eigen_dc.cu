@@ -302,20 +302,31 @@ __global__ void __launch_bounds__(256) copy_max_kernel(const double* __restrict_
   atomicMax(big, (unsigned long long)__double_as_longlong(m));
 }
 
-// Rows n .. n8 - 1 of the working copy are zero (the panels read them).  Where its
-// largest entry is beyond 2^+-RANGE the copy is multiplied by 2^*shift (LAPACK dsyevd
-// scales by the norm): reflectors and updates take products of three entries.
-__global__ void __launch_bounds__(256) scale_pad_kernel(double* __restrict__ B, long long ldb, int n,
-                                                        int n8, const unsigned long long* big,
-                                                        int* shift) {
-  const int k = range_shift(__longlong_as_double((long long)*big));
+// Clears the reflectors V, the panel W (NB columns) and rows n .. n8 - 1 of the working
+// copy (the panels read them).  Where the copy's largest entry is beyond 2^+-RANGE, it
+// is multiplied by 2^*shift (LAPACK dsyevd scales by the norm): reflectors and updates
+// take products of three entries.
+__global__ void __launch_bounds__(256) clear_scale_kernel(double* __restrict__ B, long long ldb,
+                                                          int n, int n8, double* __restrict__ V,
+                                                          long long ldv, double* __restrict__ W,
+                                                          long long ldw,
+                                                          const unsigned long long* big,
+                                                          int* shift) {
+  const int k = range_shift(__longlong_as_double((long long)*big)), tid = threadIdx.x;
+  const double2 zero = make_double2(0.0, 0.0);
   for (int c = blockIdx.x; c < n; c += gridDim.x) {
     double* b = B + (long long)c * ldb;
-    if (n + (int)threadIdx.x < n8) b[n + threadIdx.x] = 0.0;
+    if (n + tid < n8) b[n + tid] = 0.0;
     if (k != 0)
-      for (int r = threadIdx.x; r < n; r += 256) b[r] = scalbn(b[r], k);
+      for (int r = tid; r < n; r += 256) b[r] = scalbn(b[r], k);
+    double2* v = (double2*)(V + (long long)c * ldv);
+    for (int r = tid; 2 * r < ldv; r += 256) v[r] = zero;
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0) *shift = k;
+  for (int c = blockIdx.x; c < NB; c += gridDim.x) {
+    double2* w = (double2*)(W + (long long)c * ldw);
+    for (int r = tid; 2 * r < ldw; r += 256) w[r] = zero;
+  }
+  if (blockIdx.x == 0 && tid == 0) *shift = k;
 }
 
 // The eigenvalues of the matrix as it was.
@@ -1378,11 +1389,10 @@ int eigen_dc(imcom_ctx* ctx, const DMat& A, DMat& Wout, double* wout) {
     const unsigned grid = (unsigned)std::min(n, 8 * sm_count(ctx));
     copy_max_kernel<<<grid, 256, 0, ctx->stream>>>(A.p, A.ld, Aw.p, Aw.ld, n, big);
     IMC_LAUNCH();
-    scale_pad_kernel<<<grid, 256, 0, ctx->stream>>>(Aw.p, Aw.ld, n, (n + 7) & ~7, big, derr + 2);
+    clear_scale_kernel<<<grid, 256, 0, ctx->stream>>>(Aw.p, Aw.ld, n, (n + 7) & ~7, Vall.p,
+                                                      Vall.ld, Wp, ldw, big, derr + 2);
     IMC_LAUNCH();
   }
-  IMC_CUDA(cudaMemsetAsync(Vall.p, 0, Vall.bytes(), ctx->stream));
-  IMC_CUDA(cudaMemsetAsync(Wp, 0, (size_t)ldw * NB * 8, ctx->stream));
   if (two)
     IMC_TRY(twostage_tridiag(ctx, Aw, Vall, d, e, tau, Wp, ldw, (double*)(base + o_XY),
                              base + o_2s, spin));
