@@ -453,13 +453,21 @@ static int build_images(imcom_ctx* ctx, int nstack, const double* dI, long long 
   // 800, 128 stacks (4.2e8 products), 76 / 73 at m = 1200, 96 stacks (4.7e8),
   // 223 / 178 at m = 4096, 128 stacks; the other way round 41 / 53 at n =
   // 1000, m = 1500, 192 stacks (2.9e8).
-  if (ctx->stack_kernel == IMCOM_STACKS_AUTO &&
-      (nstack <= 64 || (double)ctx->n * ctx->m * nstack <= 3e8)) {
+  // The streaming kernel keeps one stack where m gives it warps enough (tensor /
+  // streaming, us a call: 20.3 / 15.7 at n = m = 2000, 15.6 / 13.6 at 1453 x 529, 16.6 /
+  // 19.5 at 3000 x 700) and 17 to 32 stacks of small problems, whose sums the tensor
+  // kernel splits (25.6 / 22.1 at 1000 x 1500, 32 stacks; 19.6 / 23.9 at 1500 x 1000,
+  // 17.4 / 23.6 at 512 x 2500).
+  const int n = ctx->n, m = ctx->m;
+  const bool few = (nstack == 1 && n <= 4LL * m) ||
+                   (nstack > 16 && nstack <= 32 && n <= 1200 && m <= 1600);
+  const bool automatic = ctx->stack_kernel == IMCOM_STACKS_AUTO;
+  if (automatic && !few && (nstack <= 64 || (double)n * m * nstack <= 3e8)) {
     IMC_TRY(stacks_mma(ctx, nstack, dI, ldi, dH, ldh));
     stage_end(ctx, ST_EPI);
     return 0;
   }
-  const bool stream = ctx->stack_kernel == IMCOM_STACKS_STREAM;
+  const bool stream = ctx->stack_kernel == IMCOM_STACKS_STREAM || (automatic && few);
   if (stream) {
     // passes of at most 8 stacks: 4 x 8 partial sums and two 4 x 4 blocks of
     // T values per lane fill the register budget of three CTAs per SM

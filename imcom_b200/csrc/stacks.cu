@@ -2,25 +2,28 @@
 // (imcom_build_image, imcom_matrix.f90:754-790, for S stacks that share T).
 //
 // T (n x m) and the stacks (n x S) are both contiguous along the summed
-// dimension.  A CTA owns 32 output pixels and NT stacks; its eight warps are
-// 2 (pixels) x 4 (slices of each 64-deep stage), a warp holding 16 x NT sums
-// in m16n8k4 DMMA tiles, and the four slices are added through shared memory
-// at the end.  So T crosses HBM once for up to 64 stacks, the stacks come
-// from L2, and 32 pixels per CTA give one CTA per SM at m of about 4700
-// without splitting the sum; other sizes split it over a few CTAs and add the
-// partial sums in a second kernel.
+// dimension.  A CTA owns 32 output pixels and NT stacks; each of its eight warps
+// takes an eighth of every 64-deep stage, holding 32 x NT sums in m16n8k4 DMMA
+// tiles, and the eight slices are added through shared memory at the end.  So T
+// crosses HBM once for up to 64 stacks, the stacks come from L2, and 32 pixels
+// per CTA give one CTA per SM at m of about 4700 without splitting the sum; other
+// sizes split it over a few CTAs and add the partial sums in a second kernel.
+//
+// A sum's error grows with its length, and a DMMA adds to its accumulator one
+// product at a time.  So each stage's products (8 per slice) are summed by
+// themselves and then added to the slice's sum; tiles of more than 48 stacks,
+// which have no registers for that, take a depth of 2048 at a time instead.
+// Relative error of the result against 128-bit sums, n = m = 4096 (the FMA kernel
+// and the GEMM for comparison): 3.1e-16 (4.0e-16) up to 32 stacks, 3.1e-16 (7.3e-16)
+// up to 48, 5.5e-16 (7.3e-16) up to 64; one chain per slice: 7.6e-16.
 //
 // What bounds it: HBM (one read of T) up to about 16 stacks, the FP64 tensor
-// pipe above.  The 128 x 128 GEMM tile computes 128 stacks whatever S is, and
-// the FMA kernel (solve.cu) reads T once per eight stacks and is bound by its
-// shared-memory reads.  Measured, n = m = 4096, three T in turn (402 MB), us:
-//   S        1      8     16     48     64    128
-//   GEMM   143    143    143    144    145    149
-//   FMA     22     38     73    199    274    517
-//   here  19.4   19.6   25.3   64.9   77.8    155
-// (48 stacks are 1.6 GFLOP, 45 us at the DGEMM rate.)  Issuing a stage's
-// copies before its products instead of between them: 77.0 at S = 48; twice
-// the warps: 81.7.
+// pipe and the latency of a stage above.  The 128 x 128 GEMM tile computes 128
+// stacks whatever S is, and the FMA kernel (solve.cu) reads T once per eight
+// stacks and is bound by its shared-memory reads.  Measured, n = m = 4096, three T
+// in turn (402 MB), us: 48 stacks 178 in the GEMM, 74 here (1.6 GFLOP, 45 us at the
+// DGEMM rate; 63 with one chain per slice of a 16-deep step and 1.4e-15 of error
+// where the GEMM has 1.1e-15).
 #include <algorithm>
 
 #include "common.cuh"
@@ -35,7 +38,7 @@ __global__ void splitk_reduce_kernel(const double* __restrict__ part, long long 
 namespace {
 
 constexpr int ST_THREADS = 256, ST_BM = 32, ST_BK = 64;
-constexpr int ST_WM = 2, ST_WK = 4;        // warps over pixels and over each stage's depth
+constexpr int ST_WK = 8, ST_MT = 2;        // warps, each an eighth of a stage's depth; its pixel tiles
 constexpr int ST_SK = ST_BK + 4;           // shared stride: fragment loads hit distinct banks
 constexpr int ST_KW = ST_BK / ST_WK;       // depth per warp and stage
 
@@ -47,6 +50,11 @@ constexpr int st_stage() {
 template <int NT>
 constexpr int st_stages() {
   return NT <= 32 ? 4 : 3;
+}
+// Whether each stage's products are summed by themselves first (twice the registers).
+template <int NT>
+constexpr bool st_staged() {
+  return NT <= 48;
 }
 template <int NT>
 constexpr size_t st_smem() {
@@ -65,7 +73,6 @@ stacks_mma_kernel(const double* __restrict__ T, long long ldt, const double* __r
   extern __shared__ __align__(16) double st_sm[];
   constexpr int STG = st_stages<NT>(), SZ = st_stage<NT>();
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int wm = warp & (ST_WM - 1), wk = warp / ST_WM;
   const int g = lane >> 2, t = lane & 3;
   const int a0 = blockIdx.x * ST_BM, s0 = blockIdx.y * NT;
   const int kb = blockIdx.z * kchunk, ke = min(n, kb + kchunk);
@@ -75,38 +82,42 @@ stacks_mma_kernel(const double* __restrict__ T, long long ldt, const double* __r
   I += (long long)s0 * ldi;
   if (gridDim.z > 1) H += (size_t)blockIdx.z * (size_t)ldh * (size_t)S;  // partial slice
 
-  // Quarter u of stage kt: pixel rows 8 u .. 8 u + 7 of T and every fourth
-  // group of the stacks' copies.
+  // Quarter u of stage kt: pixel rows 8 u .. 8 u + 7 of T and every fourth group of
+  // the stacks' copies.  Rows past the last one copy it again (their sums are not
+  // written), so only the last stage's depth needs a test.
   const int tr = tid / (ST_BK / 2), tk = tid % (ST_BK / 2) * 2;
-  const double* tsrc = T + (long long)tr * ldt + kb + tk;
+  const double* tsrc = T + kb + tk;
   double* tdst = st_sm + tr * ST_SK + tk;
   const int ir = tid / (ST_BK / VI), ik = tid % (ST_BK / VI) * VI;
   constexpr int IROWS = ST_THREADS / (ST_BK / VI);  // stacks per group of copies
-  const double* isrc = I + (long long)ir * ldi + kb + ik;
+  const double* isrc = I + kb + ik;
   double* idst = st_sm + (ST_BM + ir) * ST_SK + ik;
   auto load = [&](int kt, int u) {
     const int st = (kt % STG) * SZ, left = ke - kb - kt * ST_BK;
-    {
-      const int r = tr + 8 * u, l = r < na ? left - tk : 0;
-      gemm::cp_async(tdst + st + 8 * u * ST_SK,
-                     l > 0 ? tsrc + (long long)8 * u * ldt + kt * ST_BK : T,
-                     8 * max(0, min(l, 2)), 2);
-    }
+    const double* ts = tsrc + (long long)min(tr + 8 * u, na - 1) * ldt + kt * ST_BK;
+    double* td = tdst + st + 8 * u * ST_SK;
+    if (left >= ST_BK) gemm::cp_async(td, ts, 16, 2);
+    else gemm::cp_async(td, left > tk ? ts : T, 8 * max(0, min(left - tk, 2)), 2);
 #pragma unroll
     for (int q = u; q < NT / IROWS; q += 4) {
-      const int r = ir + IROWS * q, l = r < ns ? left - ik : 0;
-      gemm::cp_async(idst + st + IROWS * q * ST_SK,
-                     l > 0 ? isrc + (long long)IROWS * q * ldi + kt * ST_BK : I,
-                     8 * max(0, min(l, VI)), VI);
+      const double* is = isrc + (long long)min(ir + IROWS * q, ns - 1) * ldi + kt * ST_BK;
+      double* id = idst + st + IROWS * q * ST_SK;
+      if (left >= ST_BK) gemm::cp_async(id, is, 8 * VI, VI);
+      else gemm::cp_async(id, left > ik ? is : I, 8 * max(0, min(left - ik, VI)), VI);
     }
   };
-  static_assert(ST_BM == 32 && ST_THREADS / (ST_BK / 2) == 8 && ST_KW == 16, "quarters of a stage");
+  static_assert(ST_BM == 16 * ST_MT && ST_THREADS / (ST_BK / 2) == 8 && ST_KW == 8,
+                "quarters of a stage, two at each of a warp's two steps");
 
-  double acc[NT / 8][4];
+  // the sums, and those of the current stage
+  constexpr int R = st_staged<NT>() ? 1 : 0;
+  double sum[1 + R][ST_MT][NT / 8][4];
 #pragma unroll
-  for (int j = 0; j < NT / 8; ++j)
+  for (int i = 0; i < ST_MT; ++i)
 #pragma unroll
-    for (int r = 0; r < 4; ++r) acc[j][r] = 0.0;
+    for (int j = 0; j < NT / 8; ++j)
+#pragma unroll
+      for (int r = 0; r < 4; ++r) sum[0][i][j][r] = sum[R][i][j][r] = 0.0;
 #pragma unroll
   for (int s = 0; s < STG - 1; ++s) {
     if (s < nk)
@@ -116,42 +127,69 @@ stacks_mma_kernel(const double* __restrict__ T, long long ldt, const double* __r
   for (int kt = 0; kt < nk; ++kt) {
     gemm::cp_wait<STG - 2>();
     __syncthreads();
-    const double* sa = st_sm + (kt % STG) * SZ + (wm * 16 + g) * ST_SK + wk * ST_KW + t;
-    const double* sb = st_sm + (kt % STG) * SZ + (ST_BM + g) * ST_SK + wk * ST_KW + t;
+    const double* sa = st_sm + (kt % STG) * SZ + g * ST_SK + warp * ST_KW + t;
+    const double* sb = sa + ST_BM * ST_SK;
 #pragma unroll
     for (int kk = 0; kk < ST_KW; kk += 4) {
       // the next stage's copies between the products, which leave most issue
       // slots free
-      if (kt + STG - 1 < nk) load(kt + STG - 1, kk / 4);
-      const double f0 = sa[kk], f1 = sa[8 * ST_SK + kk];
+      if (kt + STG - 1 < nk) {
+        load(kt + STG - 1, kk / 2);
+        load(kt + STG - 1, kk / 2 + 1);
+      }
+      double f[ST_MT][2];
+#pragma unroll
+      for (int i = 0; i < ST_MT; ++i) {
+        f[i][0] = sa[16 * i * ST_SK + kk];
+        f[i][1] = sa[(16 * i + 8) * ST_SK + kk];
+      }
 #pragma unroll
       for (int j = 0; j < NT / 8; ++j) {
         const double b = sb[8 * j * ST_SK + kk];
-        asm volatile(
-            "mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5}, {%6}, "
-            "{%0,%1,%2,%3};\n"
-            : "+d"(acc[j][0]), "+d"(acc[j][1]), "+d"(acc[j][2]), "+d"(acc[j][3])
-            : "d"(f0), "d"(f1), "d"(b));
+#pragma unroll
+        for (int i = 0; i < ST_MT; ++i) {
+          double* c = sum[R][i][j];
+          asm volatile(
+              "mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5}, {%6}, "
+              "{%0,%1,%2,%3};\n"
+              : "+d"(c[0]), "+d"(c[1]), "+d"(c[2]), "+d"(c[3])
+              : "d"(f[i][0]), "d"(f[i][1]), "d"(b));
+        }
       }
     }
     gemm::cp_commit();
+    if (R) {
+#pragma unroll
+      for (int i = 0; i < ST_MT; ++i)
+#pragma unroll
+        for (int j = 0; j < NT / 8; ++j)
+#pragma unroll
+          for (int r = 0; r < 4; ++r) {
+            sum[0][i][j][r] += sum[R][i][j][r];
+            sum[R][i][j][r] = 0.0;
+          }
+    }
   }
   gemm::cp_wait<0>();
   __syncthreads();
-  // the four depth slices' sums, [slice][pixel][stack]
-  double* sums = st_sm + (size_t)wk * ST_BM * (NT + 1);
+  // the depth slices' sums, [slice][pixel][stack]
+  double* sums = st_sm + (size_t)warp * ST_BM * (NT + 1);
 #pragma unroll
-  for (int j = 0; j < NT / 8; ++j)
+  for (int i = 0; i < ST_MT; ++i)
 #pragma unroll
-    for (int r = 0; r < 4; ++r)
-      sums[(wm * 16 + g + ((r >> 1) ? 8 : 0)) * (NT + 1) + 8 * j + 2 * t + (r & 1)] = acc[j][r];
+    for (int j = 0; j < NT / 8; ++j)
+#pragma unroll
+      for (int r = 0; r < 4; ++r)
+        sums[(16 * i + g + ((r >> 1) ? 8 : 0)) * (NT + 1) + 8 * j + 2 * t + (r & 1)] =
+            sum[0][i][j][r];
   __syncthreads();
   for (int e = tid; e < ST_BM * NT; e += ST_THREADS) {
     const int r = e % ST_BM, s = e / ST_BM;
     if (r < na && s < ns) {
       const double* p = st_sm + r * (NT + 1) + s;
       constexpr int Z = ST_BM * (NT + 1);
-      H[(a0 + r) + (long long)(s0 + s) * ldh] = (p[0] + p[Z]) + (p[2 * Z] + p[3 * Z]);
+      H[(a0 + r) + (long long)(s0 + s) * ldh] = ((p[0] + p[Z]) + (p[2 * Z] + p[3 * Z])) +
+                                                ((p[4 * Z] + p[5 * Z]) + (p[6 * Z] + p[7 * Z]));
     }
   }
 }
@@ -174,6 +212,8 @@ int launch_nt(imcom_ctx* ctx, int S, const double* dI, long long ldi, double* dH
       splits = s;
     }
   }
+  // (tiles that do not sum each stage by itself take a depth of 2048 at a time)
+  if (!st_staged<NT>()) splits = std::max(splits, (n + 2047) / 2048);
   const int kchunk = (ksteps + splits - 1) / splits * ST_BK;
   splits = (n + kchunk - 1) / kchunk;
   double* out = dH;
