@@ -63,24 +63,24 @@ constexpr size_t st_smem() {
   return (pipe > sums ? pipe : sums) * sizeof(double);
 }
 
-// VI: doubles per copy of the stacks (2 where their columns are 16-byte
-// aligned, else 1); T's columns always are.
+// Tile (bx, by) of slice bz of nz of the sum.  VI: doubles per copy of the stacks (2
+// where their columns are 16-byte aligned, else 1); T's columns always are.
 template <int NT, int VI>
-__global__ void __launch_bounds__(ST_THREADS)
-stacks_mma_kernel(const double* __restrict__ T, long long ldt, const double* __restrict__ I,
-                  long long ldi, double* __restrict__ H, long long ldh, int n, int m, int S,
-                  int kchunk) {
+__device__ __forceinline__ void stacks_tile(const double* __restrict__ T, long long ldt,
+                                            const double* __restrict__ I, long long ldi,
+                                            double* __restrict__ H, long long ldh, int n, int m,
+                                            int S, int kchunk, int bx, int by, int bz, int nz) {
   extern __shared__ __align__(16) double st_sm[];
   constexpr int STG = st_stages<NT>(), SZ = st_stage<NT>();
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int g = lane >> 2, t = lane & 3;
-  const int a0 = blockIdx.x * ST_BM, s0 = blockIdx.y * NT;
-  const int kb = blockIdx.z * kchunk, ke = min(n, kb + kchunk);
+  const int a0 = bx * ST_BM, s0 = by * NT;
+  const int kb = bz * kchunk, ke = min(n, kb + kchunk);
   const int nk = (ke - kb + ST_BK - 1) / ST_BK;
   const int na = min(ST_BM, m - a0), ns = min(NT, S - s0);
   T += (long long)a0 * ldt;
   I += (long long)s0 * ldi;
-  if (gridDim.z > 1) H += (size_t)blockIdx.z * (size_t)ldh * (size_t)S;  // partial slice
+  if (nz > 1) H += (size_t)bz * (size_t)ldh * (size_t)S;  // partial slice
 
   // Quarter u of stage kt: pixel rows 8 u .. 8 u + 7 of T and every fourth group of
   // the stacks' copies.  Rows past the last one copy it again (their sums are not
@@ -194,6 +194,28 @@ stacks_mma_kernel(const double* __restrict__ T, long long ldt, const double* __r
   }
 }
 
+template <int NT, int VI>
+__global__ void __launch_bounds__(ST_THREADS)
+stacks_mma_kernel(const double* __restrict__ T, long long ldt, const double* __restrict__ I,
+                  long long ldi, double* __restrict__ H, long long ldh, int n, int m, int S,
+                  int kchunk) {
+  stacks_tile<NT, VI>(T, ldt, I, ldi, H, ldh, n, m, S, kchunk, blockIdx.x, blockIdx.y, blockIdx.z,
+                      gridDim.z);
+}
+
+// The same tiles, gx x gy x gz of them, in turn on the CTAs of a share of the SMs.
+template <int NT, int VI>
+__global__ void __launch_bounds__(ST_THREADS)
+stacks_share_kernel(const double* __restrict__ T, long long ldt, const double* __restrict__ I,
+                    long long ldi, double* __restrict__ H, long long ldh, int n, int m, int S,
+                    int kchunk, int gx, int gy, int gz) {
+  for (int b = blockIdx.x; b < gx * gy * gz; b += gridDim.x) {
+    __syncthreads();  // every warp is done with the previous tile's shared memory
+    stacks_tile<NT, VI>(T, ldt, I, ldi, H, ldh, n, m, S, kchunk, b % gx, b / gx % gy, b / gx / gy,
+                        gz);
+  }
+}
+
 template <int NT>
 int launch_nt(imcom_ctx* ctx, int S, const double* dI, long long ldi, double* dH, long long ldh) {
   const int n = ctx->n, m = ctx->m, sms = sm_count(ctx);
@@ -225,13 +247,26 @@ int launch_nt(imcom_ctx* ctx, int S, const double* dI, long long ldi, double* dH
     out = (double*)ctx->gemm_ws;
   }
   const bool v2 = ((uintptr_t)dI & 15) == 0 && ldi % 2 == 0;
-  auto k = v2 ? stacks_mma_kernel<NT, 2> : stacks_mma_kernel<NT, 1>;
-  IMC_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)st_smem<NT>()));
-  const dim3 grd((unsigned)((m + ST_BM - 1) / ST_BM), (unsigned)((S + NT - 1) / NT),
-                 (unsigned)splits);
-  k<<<grd, ST_THREADS, st_smem<NT>(), ctx->stream>>>(ctx->T.p, ctx->T.ld, dI, ldi, out, ldo, n, m,
-                                                     S, kchunk);
+  const int gx = (m + ST_BM - 1) / ST_BM, gy = (S + NT - 1) / NT;
+  const size_t smem = st_smem<NT>();
+  // on a share of the SMs, products bound by the tensor pipe keep to it: one CTA per
+  // SM, as the GEMM (few stacks are bound by the read of T)
+  bool done = false;
+  if constexpr (NT > 32) {
+    if (ctx->sm_share > 0) {
+      auto k = v2 ? stacks_share_kernel<NT, 2> : stacks_share_kernel<NT, 1>;
+      IMC_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      k<<<(unsigned)std::min<long long>(tiles * splits, sms), ST_THREADS, smem, ctx->stream>>>(
+          ctx->T.p, ctx->T.ld, dI, ldi, out, ldo, n, m, S, kchunk, gx, gy, splits);
+      done = true;
+    }
+  }
+  if (!done) {
+    auto k = v2 ? stacks_mma_kernel<NT, 2> : stacks_mma_kernel<NT, 1>;
+    IMC_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    k<<<dim3((unsigned)gx, (unsigned)gy, (unsigned)splits), ST_THREADS, smem, ctx->stream>>>(
+        ctx->T.p, ctx->T.ld, dI, ldi, out, ldo, n, m, S, kchunk);
+  }
   IMC_LAUNCH();
   if (splits > 1) {
     const dim3 g2((unsigned)std::min((m + 255) / 256, 64), (unsigned)S);
