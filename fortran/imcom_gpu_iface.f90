@@ -266,7 +266,7 @@ INTERFACE
   END FUNCTION
 
   ! imcom_build_image for nstack image stacks sharing the resident T:
-  ! I_stack(n, nstack) -> H(m, nstack), one FP64 GEMM (T read once)
+  ! I_stack(n, nstack) -> H(m, nstack), one FP64 product (T read once)
   INTEGER(C_INT) FUNCTION imcom_gpu_build_images(ctx, nstack, I_stack, H) &
                                                  BIND(C, NAME="imcom_gpu_build_images")
     IMPORT :: C_INT, C_PTR, C_DOUBLE

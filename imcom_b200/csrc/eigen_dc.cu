@@ -473,7 +473,7 @@ __global__ void __launch_bounds__(256) leaf_jacobi_kernel(const Node* nodes, con
           Am[pi][qj] = own ? 0.0 : ci * bpq - si * bqq;
           Am[qi][pj] = own ? 0.0 : si * bpp + ci * bqp;
           Am[qi][qj] = si * bpq + ci * bqq;
-          // rows i and i + NP of Z
+          // rows i and i + mp / 2 of Z
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
             const int r = i + h * (mp / 2);
@@ -1238,7 +1238,7 @@ static int sytrd_launches(imcom_ctx* ctx, DMat& Aw, DMat& Vall, double* d, doubl
       int h = 0;
       IMC_CUDA(cudaMemcpyAsync(&h, err, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
       IMC_CUDA(cudaStreamSynchronize(ctx->stream));
-      if (h) return set_err(ctx, IMCOM_ERR_EIGEN, "tridiagonalisation grid barrier timed out");
+      if (h) return set_err(ctx, IMCOM_ERR_EIGEN, "a wait of the tridiagonalisation timed out (exchange or barrier)");
     }
   }
   if (!tail_done) {  // the tail writes the last diagonal entry itself
@@ -1407,7 +1407,7 @@ int eigen_dc(imcom_ctx* ctx, const DMat& A, DMat& Wout, double* wout) {
     int h[3] = {};
     IMC_CUDA(cudaMemcpyAsync(h, derr, sizeof h, cudaMemcpyDeviceToHost, ctx->stream));
     IMC_CUDA(cudaStreamSynchronize(ctx->stream));
-    if (h[1]) return set_err(ctx, IMCOM_ERR_EIGEN, "tridiagonalisation grid barrier timed out");
+    if (h[1]) return set_err(ctx, IMCOM_ERR_EIGEN, "a wait of the tridiagonalisation timed out (exchange or barrier)");
     if (h[0])
       return set_err(ctx, IMCOM_ERR_EIGEN, "the tridiagonal matrix has a non-finite entry");
     shift = h[2];

@@ -34,7 +34,8 @@
 // per column of exchanges and sums.  Microseconds per column with the trailing
 // update, before (grid barriers, tiles through shared memory) and now: from
 // 8192 to 2048 rows 43.8 -> 32.9, from 4096 18.5 -> 12.6, from 3000 19.1 -> 11.0,
-// from 1453 down 8.5 -> 7.4, from 512 down 7.7 -> 8.1.  Row sums that wait for the
+// from 1453 down 8.5 -> 7.4, from 512 down 8.1 either way (8.0 to 8.2 by machine; 16 to
+// 32 CTAs there instead of all: 7.9).  Row sums that wait for the
 // reflector's scalars before they go out cost 1.2 us per column more; dots
 // laid out by sum and not by CTA (lines that eight CTAs write), 0.6; fewer rows
 // per owner than a warp has lanes (16 at 2100 rows), 0.5.

@@ -93,8 +93,9 @@ typedef struct imcom_ctx imcom_ctx;
 #define IMCOM_OPT_SM_SHARE 10
 /* How the tridiagonalisation ends: 0 (default) = the trailing matrix resident
  * in the shared memory of this context's SMs (up to order 2048 on 148 SMs),
- * one exchange per column (a share below 8 SMs: the cluster); 8 or 16 = a thread-block cluster of that many
- * CTAs (8 if 16 cannot be placed) once the trailing matrix fits its
+ * one exchange per column (a share below 8 SMs: the cluster); 8 or 16 = a
+ * thread-block cluster of that many CTAs (8 if 16 cannot be placed) once the
+ * trailing matrix fits its
  * distributed shared memory; -1 = panels to the end.  A 16-CTA cluster must
  * find 16 free SMs in one GPC, which contexts working side by side can make
  * wait; smaller clusters hold smaller tails.  Same results to rounding
@@ -103,15 +104,16 @@ typedef struct imcom_ctx imcom_ctx;
 /* Kernel of imcom_gpu_build_images: 0 = the FP64 GEMM, 1 = a streaming
  * kernel for a few stacks (up to 8 stacks per pass over T, FP64 FMA, each
  * warp holding four columns of T against the stacks of its pass), 2 (default)
- * = an FP64 tensor-core kernel with 32-pixel tiles for up to 64 stacks (and
- * for more where the product is small), the GEMM above.  Same sums to
- * rounding. */
+ * = the streaming kernel for one stack (unless n > 4 m) and for 17 to 32 stacks
+ * of small problems (n <= 1200, m <= 1600), else an FP64 tensor-core kernel with
+ * 32-pixel tiles for up to 64 stacks (and for more where the product is small),
+ * the GEMM above.  Same sums to rounding. */
 #define IMCOM_OPT_STACK_KERNEL 12
 #define IMCOM_STACKS_GEMM 0
 #define IMCOM_STACKS_STREAM 1
 #define IMCOM_STACKS_AUTO 2
-#define IMCOM_STACKS_STREAM_MAX 32 /* stacks beyond which the streaming kernel loses
-                                   to the GEMM */
+#define IMCOM_STACKS_STREAM_MAX 32 /* for callers that choose: stacks beyond which the
+                                   streaming kernel loses to the GEMM */
 /* Inverse 2-D FFT of the lookup tables (imcom_build_Alookup/Blookup): 0 =
  * embedding, cuFFT and shift as separate steps; 1 = the library's own
  * transform in two passes that skip the grid's zero lines and fuse the

@@ -1,6 +1,6 @@
 """CPU oracle of the learned-kappa MLP training step (test infrastructure only).
 
-numpy restatement of imcom_b200/csrc/kappa.cu's mlp_grad_kernel: the same
+numpy restatement of imcom_b200/csrc/kappa.cu's mlp_train_kernel: the same
 bf16 rounding points (inputs, weights, hidden activations; round to nearest
 even), ReLU masks taken on the rounded activations, the same loss
 (o0 - t)^2 + 0.25 (o1 - log(|o0 - t| + 0.01))^2 with the second target held
