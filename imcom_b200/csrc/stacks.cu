@@ -20,10 +20,14 @@
 // What bounds it: HBM (one read of T) up to about 16 stacks, the FP64 tensor
 // pipe and the latency of a stage above.  The 128 x 128 GEMM tile computes 128
 // stacks whatever S is, and the FMA kernel (solve.cu) reads T once per eight
-// stacks and is bound by its shared-memory reads.  Measured, n = m = 4096, three T
-// in turn (402 MB), us: 48 stacks 178 in the GEMM, 74 here (1.6 GFLOP, 45 us at the
-// DGEMM rate; 63 with one chain per slice of a 16-deep step and 1.4e-15 of error
-// where the GEMM has 1.1e-15).
+// stacks and is bound by its shared-memory reads.  Measured, 48 stacks at 3999 x
+// 4225, us: 178 in the GEMM, 74 here (1.6 GFLOP, 45 us at the DGEMM rate; 63 with one
+// chain per slice of a 16-deep step and 1.4e-15 of error where the GEMM has 1.1e-15).
+// n = m = 4096 in a loop of calls, us a call:
+//   S          2     8    16    32    48    64
+//   GEMM     169   169   169   169   169   169
+//   FMA       52    69   113   190
+//   here      39    36    48    71    91   110
 #include <algorithm>
 
 #include "common.cuh"
