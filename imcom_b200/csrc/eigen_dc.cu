@@ -270,7 +270,8 @@ __device__ __forceinline__ int range_shift(double mag) {
 }
 
 // The working copy of A, and the bits of the largest magnitude in its lower triangle
-// (zero before).
+// (zero before).  Bound by HBM: 40 us at n = 4096 (268 MB); 3.6 us at 72, as the copy
+// alone was.
 __global__ void __launch_bounds__(256) copy_max_kernel(const double* __restrict__ A, long long lda,
                                                        double* __restrict__ B, long long ldb,
                                                        int n, unsigned long long* big) {
@@ -305,7 +306,8 @@ __global__ void __launch_bounds__(256) copy_max_kernel(const double* __restrict_
 // Clears the reflectors V, the panel W (NB columns) and rows n .. n8 - 1 of the working
 // copy (the panels read them).  Where the copy's largest entry is beyond 2^+-RANGE, it
 // is multiplied by 2^*shift (LAPACK dsyevd scales by the norm): reflectors and updates
-// take products of three entries.
+// take products of three entries.  Bound by the write of V, as the memset that it
+// stands for; 3.2 us at n = 72, 5.3 at 1453.
 __global__ void __launch_bounds__(256) clear_scale_kernel(double* __restrict__ B, long long ldb,
                                                           int n, int n8, double* __restrict__ V,
                                                           long long ldv, double* __restrict__ W,
@@ -343,7 +345,8 @@ struct Node {
 };
 
 // dt = d, and bit 16 of *err where d or e is not finite (a matrix that is not, or
-// whose reduction overflowed): nothing below runs on such values.
+// whose reduction overflowed): nothing below runs on such values.  One CTA, so that one
+// word is written: 2.8 us at n = 72, 4.7 at 1453.
 __global__ void __launch_bounds__(1024) dc_input_kernel(const double* d, const double* e, int n,
                                                         double* dt, int* err) {
   bool bad = false;
